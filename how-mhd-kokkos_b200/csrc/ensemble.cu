@@ -271,6 +271,7 @@ int build_sweep_tables(how_ensemble* e) {
                     a.ctb = c.ct[ct_b[d]];
                     a.dtdl = &c.dsc->dtdl[iw][d];
                     a.gam = c.p.gam; a.rhomin = c.p.rhomin; a.pgmin = c.p.pgmin;
+                    a.gam2 = (a.gam - 2.0) / (a.gam - 1.0);
                     a.ct4 = c.p.ct_avg == 4;
                     a.status = e->d_status;
                     const int bin = phys_stage(par, iw - 1);

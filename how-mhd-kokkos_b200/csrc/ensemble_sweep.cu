@@ -1,7 +1,7 @@
 // ensemble_sweep.cu -- the fused sweep over every member of a batched
-// ensemble in one persistent launch, for each tile shape the autotuner may
-// pick.  Member m's tiles occupy [tile_start[m], tile_start[m+1]) of the
-// launch's tile space; each tile reads its member's arguments (geometry,
+// ensemble in one persistent launch, for each work-item shape the autotuner
+// may pick.  Member m's items occupy [tile_start[m], tile_start[m+1]) of the
+// launch's item space; each item reads its member's arguments (geometry,
 // stage pointers, TMA tensor maps, dt) from a device table.
 #include "sweep_core.cuh"
 #include "ensemble.cuh"
@@ -10,80 +10,79 @@ namespace how {
 
 namespace {
 
-// Candidate tile shapes (lines x active cells) per direction.  y/z lines are
-// consecutive i from an even start, so NL is even there (16-byte TMA rule).
-struct ShapeDef { int nl, t, minb; };
+// Candidate shapes per direction: lines per warp and chunks per work item
+// (k_sweep).  Short items spread small members over the chip, long ones repeat
+// less work at segment ends; one line per warp suits 1-D members.  y/z lines
+// are consecutive i and NL is even there (16-byte TMA rule).
+struct ShapeDef { int nl, chunks; };
 constexpr ShapeDef kShapes[3][kEnsShapes] = {
-    {{1, 32, 4}, {1, 64, 2}, {2, 16, 4}},
-    {{2, 16, 4}, {2, 32, 2}, {4, 8, 4}},
-    {{2, 16, 4}, {2, 16, 4}, {2, 16, 4}},
+    {{4, 2}, {4, 8}, {1, 2}},
+    {{4, 2}, {4, 8}, {2, 2}},
+    {{4, 2}, {4, 8}, {4, 4}},
 };
+constexpr int kWarps = 4, kBlocks = 2;   // warps per block, blocks per SM: as the single-domain FP64 sweep
 
-template <int DIR, int NL, int T, int MINB>
-void launch_ens(const SweepArgs& a0, cudaStream_t st, int dev) {
-    using TL = Tile<DIR, NL, T, double>;
-    constexpr size_t bytes = TL::bytes_plain + 128;
-    auto kern = k_sweep<DIR, NL, T, 128, double, MINB, 0, true>;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        attr_done = true;
+template <int DIR, int NL>
+void launch_ens(SweepArgs a0, int chunks, cudaStream_t st, int dev) {
+    constexpr int bytes = kWarps * WarpMem<DIR, NL, double, 0>::bytes + 128;
+    const auto kern = k_sweep<DIR, NL, kWarps, double, kBlocks, 0, true>;
+    static const int resident = [&] {
+        int nsm = 148, occ = 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * kWarps, bytes);
+        return nsm * (occ < 1 ? 1 : occ);
+    }();
+    a0.seg_chunks = chunks;
+    kern<<<resident, 32 * kWarps, bytes, st>>>(a0);
+}
+
+template <int DIR>
+long long items_of(const Grid& g, const ShapeDef& d) {
+    switch (d.nl) {
+        case 1: return Cut<DIR, 1>(g, d.chunks).items();
+        case 2: return Cut<DIR, 2>(g, d.chunks).items();
+        default: return Cut<DIR, 4>(g, d.chunks).items();
     }
-    int nsm = 148, occ = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 128, bytes);
-    if (occ < 1) occ = 1;
-    kern<<<nsm * occ, 128, bytes, st>>>(a0);
 }
 
 }  // namespace
 
+// (lines, cells a work item advances along the sweep)
 void ens_shape(int dir, int s, int* nl, int* t) {
-    *nl = kShapes[dir][s].nl;
-    *t = kShapes[dir][s].t;
+    const ShapeDef& d = kShapes[dir][s];
+    *nl = d.nl;
+    *t = d.chunks * (32 / d.nl) - (dir == 0 ? 2 : 1);
 }
 
 long long ens_tiles(const Grid& g, int dir, int s) {
-    const int NL = kShapes[dir][s].nl, T = kShapes[dir][s].t;
     const int n = dir == 0 ? g.nx : dir == 1 ? g.ny : g.nz;
     if (n <= 1) return 0;
-    const int nt1 = dir == 0 ? g.ny : g.nx;
-    const int nt2 = dir == 2 ? g.ny : g.nz;
-    const long long ntx = (n + T - 1) / T;
-    const long long nty = dir == 0 ? (nt1 + NL - 1) / NL : (nt1 + 1 + NL - 1) / NL;
-    return ntx * nty * nt2;
+    const ShapeDef& d = kShapes[dir][s];
+    return dir == 0 ? items_of<0>(g, d) : dir == 1 ? items_of<1>(g, d) : items_of<2>(g, d);
 }
 
 // Tensor maps of the 6 stage buffers of a context for shape s of direction dir.
 int ens_encode_maps(const Ctx& c, int dir, int s, CUtensorMap* tm_in, CUtensorMap* tm_out) {
-    const int NL = kShapes[dir][s].nl, T = kShapes[dir][s].t;
-    const int C = T + 6, TO = dir == 0 ? T + 2 : T;
-    const Grid& g = c.g;
-    const uint64_t dims[4] = {(uint64_t)g.P0, (uint64_t)g.P1, (uint64_t)g.P2, 8};
-    const uint64_t strides[3] = {(uint64_t)g.pitch * 8, (uint64_t)g.pitch * g.P1 * 8, (uint64_t)g.fs * 8};
-    uint32_t bin[4], bout[4];
-    if (dir == 0) { bin[0] = C; bin[1] = NL; bin[2] = 1; bout[0] = TO; bout[1] = NL; bout[2] = 1; }
-    else if (dir == 1) { bin[0] = NL; bin[1] = C; bin[2] = 1; bout[0] = NL; bout[1] = TO; bout[2] = 1; }
-    else { bin[0] = NL; bin[1] = 1; bin[2] = C; bout[0] = NL; bout[1] = 1; bout[2] = TO; }
-    bin[3] = 8; bout[3] = 8;
+    const int nl = kShapes[dir][s].nl, w = 32 / nl;
     for (int b = 0; b < 6; ++b) {
-        int rc = encode_tensor_map_4d(&tm_in[b], c.qbuf[b], dims, strides, bin);
-        if (!rc) rc = encode_tensor_map_4d(&tm_out[b], c.qbuf[b], dims, strides, bout);
+        const int rc = encode_sweep_maps(c.g, dir, nl, w, dir == 0 ? w + 2 : w, c.qbuf[b], &tm_in[b], &tm_out[b]);
         if (rc) return rc;
     }
     return 0;
 }
 
 void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int dev) {
-#define HOW_ENS_CASE(D, S)                                                                             \
-    if (dir == D && s == S) {                                                                          \
-        launch_ens<D, kShapes[D][S].nl, kShapes[D][S].t, kShapes[D][S].minb>(a0, st, dev);             \
-        return;                                                                                        \
+    const ShapeDef& d = kShapes[dir][s];
+    if (dir == 0) {
+        if (d.nl == 1) launch_ens<0, 1>(a0, d.chunks, st, dev);
+        else launch_ens<0, 4>(a0, d.chunks, st, dev);
+    } else if (dir == 1) {
+        if (d.nl == 2) launch_ens<1, 2>(a0, d.chunks, st, dev);
+        else launch_ens<1, 4>(a0, d.chunks, st, dev);
+    } else {
+        launch_ens<2, 4>(a0, d.chunks, st, dev);
     }
-    HOW_ENS_CASE(0, 0) HOW_ENS_CASE(0, 1) HOW_ENS_CASE(0, 2)
-    HOW_ENS_CASE(1, 0) HOW_ENS_CASE(1, 1) HOW_ENS_CASE(1, 2)
-    if (dir == 2) launch_ens<2, kShapes[2][0].nl, kShapes[2][0].t, kShapes[2][0].minb>(a0, st, dev);
-#undef HOW_ENS_CASE
 }
 
 }  // namespace how

@@ -109,6 +109,8 @@ struct SweepArgs {
     int stage5;            // base = q0 + c4 q2 + c5 q3
     int ct4;               // 4-point face average of B_n v_t in the CT terms (else 2-point)
     double gam, rhomin, pgmin;
+    double gam2;           // (gam - 2) / (gam - 1)
+    int seg_chunks;        // length of a work item along the sweep (k_sweep's chunks)
     unsigned long long* prof;   // optional per-phase cycle counters (instrumentation)
     unsigned int* status;       // device status word (HOW_STATUS_* bits)
     // learned routing (MODE 1/2) and label collection (MODE 3)
@@ -220,6 +222,9 @@ void launch_faceb_base(Ctx& c, int iw, double c4, double c5, int stage5);
 void launch_prot(Ctx& c, int stage);
 void launch_stage5_base(Ctx& c, double c4, double c5);
 int make_sweep_tensor_maps(Ctx& c);
+// the sweep's tensor maps of one stage buffer: raw tile and update operand
+int encode_sweep_maps(const Grid& g, int dir, int lines, int cells, int op_cells, const double* buf, CUtensorMap* in,
+                      CUtensorMap* out);
 void launch_copy_fields(Ctx& c, double* dst, const double* src, int nfields);
 
 // asynchronous dump files (output.cu): join the writer, free its buffers

@@ -5,49 +5,51 @@
 //
 // The reference runs a sweep as six all-line kernels with workspaces in
 // memory (qx, ux, ax, Fx and the 7x7 L and R per interface: ~18 GB at 256^3).
-// Here one thread block owns a pencil tile of NL lines x T active cells and
-// keeps every intermediate in shared memory; HBM sees only the stage input,
-// the RK base, the stage output and the two CT flux arrays.
+// Here a warp owns NL neighbouring lines and marches along the sweep in
+// chunks of W = 32 / NL cells, one new cell and one interface per lane; HBM
+// sees only the stage input, the RK base, the stage output and the two CT
+// flux arrays.
 //
-// Phases of one block (tile cells c in [0, T+6), interfaces f in [0, T]; the
-// interface f sits between tile cells f+2 and f+3 and its WENO stencil is
-// cells f..f+5, src/ssprk.cpp:861-865):
-//   P0  the 8 conserved variables of the tile (with its 3-cell halo) and the
-//       update's read operand arrive by TMA tensor loads issued one tile
-//       ahead: blocks are persistent and double-buffer the tiles, so the
-//       HBM latency of tile n+1 hides behind the arithmetic of tile n.  The
-//       variable permutation of the y/z sweeps (src/ssprk.cpp:1054-1061,
-//       1145-1152) is applied when the tile is read from shared memory.
-//   P1  per cell: primitives with floors (458-516), eigenvalues and fluxes
-//       (538-595)
-//   P1b per cell: differences dU(c) = U(c+1) - U(c) of (F, q_proj)
-//   P2a per interface: arithmetic-mean state and the eigen-system scalars
-//       (610-660)
-//   P3  per (interface, characteristic field m): the left-eigenvector row m,
-//       built in registers from the interface's scalars
-//       (662-726, 789-818), projection of the stencil's 5 cell differences,
-//       LLF split, WENO5-JS flux (841-937).  Seven threads of a warp share an
-//       interface and read the same cells and scalars, so the shared-memory
-//       loads broadcast (below five blocks per SM a thread takes two
-//       interfaces and reuses 4 of their 6 differences).  The
-//       central part's F_{i} share is not projected: with R L = I it is added
-//       back in physical space in P4.
-//   P4  per (interface, flux component r): row r of the right-eigenvector
-//       matrix, built in registers from the scalars (729-818), the
-//       back-projection sum_m R(r,m) F^_m in m order (941-943), CT terms
-//       (967-994) stored straight to the CT flux arrays (433-456 ...)
-//   The 7x7 eigenvector matrices are never stored: shared memory holds 21
-//   scalars per interface instead of 98 matrix entries.
-//   P5  per cell: -dtdl (F^_{i+1/2} - F^_{i-1/2}) (949-965) and the stage
-//       accumulation (405-431, 1067-1096, 1158-1187)
+// One chunk (interfaces fb .. fb+W-1 of each line; interface f sits between
+// padded cells f+2 and f+3, its WENO stencil is cells f .. f+5,
+// src/ssprk.cpp:861-865; the chunk's new cells are fb+5 .. fb+W+4):
+//   load   the new cells' 8 conserved variables arrive by a TMA tensor load
+//          issued one chunk ahead, the update's read operand by one issued at
+//          the chunk's start.  The variable permutation of the y/z sweeps
+//          (src/ssprk.cpp:1054-1061, 1145-1152) is applied on reading.
+//   cell   primitives with floors (458-516), eigenvalues and fluxes (538-595)
+//          of the lane's cell, and its differences (F, q_proj) to the cell
+//          before (by shuffle) into the warp's shared-memory window, which
+//          still holds the last cells of the chunk before.
+//   face   everything of the lane's interface in registers: arithmetic-mean
+//          state and eigen-system (610-660), projection of the 5 cell
+//          differences of the stencil, LLF split and WENO5-JS of the seven
+//          fields (841-937), back-projection (941-943), CT terms (967-994).
+//   update -dtdl (F^_{i+1/2} - F^_{i-1/2}) (949-965) and the stage
+//          accumulation (405-431, 1067-1096, 1158-1187) of the cell left of
+//          the interface; the flux before comes from the neighbouring lane.
+//
+// Why this form.  The sweep is bound by the FP64 pipe (~1,350 FP64
+// instructions per zone; 220 bytes).  A form with one block per tile and the
+// seven fields on seven threads spent more than half of its issue slots on
+// other instructions, and waited at six block barriers per tile.  Here the
+// warps share nothing, so there is no block barrier; one lane forms all
+// seven fields, so the eigenvectors' common parts are formed once (see
+// project below) and no 7x7 matrix exists in any form; and the only work done
+// twice is one interface and five cells per segment end.
+//
+// Bit-for-bit reproducibility: the arithmetic is written with explicit fma
+// calls and these translation units are compiled with -fmad=false, so every
+// instantiation (single domain, ensemble member, label collection, any NL and
+// segment length) computes the same bits.
 //
 // Precision: the kernel is a template on the working type R of the
-// eigen-system, projection and WENO arithmetic (P2a-P4's characteristic part).
-// R = double is the plain method.  R = float is the mixed-precision method:
-// primitives, cell fluxes, the physical central flux F_i, the back-projected
-// interface flux sum, the CT terms and the stage update stay FP64; the FP32
-// part only carries the characteristic upwind corrections, computed from cell
-// differences that are formed in FP64 and then rounded.
+// eigen-system, projection and WENO arithmetic.  R = double is the plain
+// method.  R = float is the mixed-precision method: primitives, cell fluxes,
+// the physical central flux F_i, the back-projected interface flux sum, the
+// CT terms and the stage update stay FP64; the FP32 part only carries the
+// characteristic upwind corrections, computed from cell differences that are
+// formed in FP64 and then rounded.
 #pragma once
 
 #include "how_internal.cuh"
@@ -60,286 +62,224 @@ namespace how {
 
 namespace {
 
-template <typename R> struct Math;
-template <> struct Math<double> {
-    using V2 = double2;
-    static __device__ __forceinline__ double sq(double x) { return sqrt(x); }
-    static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
-    static __device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
-};
-template <> struct Math<float> {
-    using V2 = float2;
-    static __device__ __forceinline__ float sq(float x) { return sqrtf(x); }
-    static __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
-    static __device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
-};
+__device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// FP64 reciprocal, square root and reciprocal square root from the hardware's
+// 20-odd-bit approximations (the PTX instructions rcp.approx.ftz.f64 and
+// rsqrt.approx.ftz.f64) and one third-order step of Householder's iteration
+// (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
+// 1970): the residual e of the approximation enters through the series
+// 1/(1-e) = 1 + e + e^2 and (1-e)^(-1/2) = 1 + e/2 + 3 e^2/8, whose next term
+// is below 2^-60.  recip and root end with the correction by the exact
+// remainder (Markstein 1990), which leaves the correctly rounded result.
+// The library's sqrt() holds the FP64 pipe for 49 cycles per warp and has a
+// latency of 250 cycles (measured on one SM); root's nine operations hold it
+// for 18.
+//
+// Nothing here branches or calls: selects stand in for the ends of the range.
+// 1 / x to about an ulp (|x| in [2^-1022, 2^1022)), and correctly rounded
+__device__ __forceinline__ double near_recip(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fm(-x, y, 1.0);
+    return fm(y, fm(e, e, e), y);
+}
+__device__ __forceinline__ double recip(double x) {
+    const double y = near_recip(x), r = fm(y, fm(-x, y, 1.0), y);
+    // 1/x lies next to a midpoint when x's significand is all ones: the result
+    // is the value above a power of two, and a tie would leave the power
+    const int ones = (__double2hiint(x) & 0xfffff) == 0xfffff && __double2loint(x) == -1;
+    return __hiloint2double(__double2hiint(r), __double2loint(r) | ones);
+}
+__device__ __forceinline__ float near_recip(float x) { return __fdividef(1.0f, x); }
+
+// 1 / sqrt(x) to about an ulp, for finite x >= 2^-1022
+__device__ __forceinline__ double root_inverse(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fm(-(x * y), y, 1.0);
+    return fm(y * e, fm(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float root_inverse(float x) { return rsqrtf(x); }
+
+// sqrt(max(0, x)), correctly rounded; an x below 2^-1022 counts as zero
+__device__ __forceinline__ double root(double x) {
+    const double y = root_inverse(x), g = x * y, r = fm(fm(-g, g, x), 0.5 * y, g);
+    const int top = __double2hiint(x);
+    return top < 0x00100000 ? 0.0 : top >= 0x7ff00000 ? x : r;
+}
+__device__ __forceinline__ float root(float x) {
+    const float y = rsqrtf(x), g = x * y, r = fm(fm(-g, g, x), 0.5f * y, g);
+    return x > 0.0f ? (x < __int_as_float(0x7f800000) ? r : x) : 0.0f;
+}
+
+// x / d, correctly rounded, given y = RN(1/d): the steps of div_const
+// (how_internal.cuh); a quotient that overflows stays infinite, and one so
+// small that its remainder is subnormal is within one unit of 2^-1074 |y|
+__device__ __forceinline__ double quot(double x, double d, double y) {
+    const double q0 = x * y, q = fm(fm(-q0, d, x), y, q0);
+    return (__double2hiint(q0) & 0x7ff00000) == 0x7ff00000 ? q0 : q;
+}
+
+// the larger of two non-negative values (doubles order like their bits)
+__device__ __forceinline__ double larger(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return __longlong_as_double(x > y ? x : y);
+}
+__device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
 
 __host__ __device__ constexpr int align_up(int x, int a) { return (x + a - 1) / a * a; }
 
-template <int DIR, int NL, int T, typename R>
-struct Tile {
-    static constexpr int C = T + 6;
-    static constexpr int F = T + 1;
-    static constexpr int NP = (F + 1) / 2;
-    static constexpr int NLC = NL * C;
-    static constexpr int NLF = NL * F;
-    static constexpr int NI = NLF | 1;              // odd interface pitch: conflict-free banks
-    // update tile: x starts one cell early so its innermost TMA coordinate is even
-    static constexpr int TO = DIR == 0 ? T + 2 : T;
-    static constexpr int NQ = 8 * NLC;              // raw tile, TMA box order [var][...]
-    static constexpr int NO = 8 * NL * TO;          // update operand tile
-    static constexpr int NS = 21;                   // eigen-system scalars per interface
-    // byte offsets (base 128-byte aligned; TMA destinations on 128 B)
-    static constexpr int bQ = 0;                                   // NBUF x [8][..] raw conserved, FP64
-    static constexpr int NBUF = 2;                                // raw tiles in flight (this + 1 ahead)
-    static constexpr int NOB = 2;                                 // update operands in flight (this + next)
-    static constexpr int bO = bQ + NBUF * align_up(8 * NQ, 128);   // NOB x [8][..] update operand, FP64
-    static constexpr int bFc = bO + NOB * align_up(8 * NO, 128);   // [NLC][7] cell fluxes, FP64
-    static constexpr int bP = bFc + align_up(8 * 7 * NLC, 16);     // [9][NLC] primitives, FP64
-    static constexpr int bA = bP + align_up(8 * 9 * NLC, 16);      // [7][NLC] eigenvalues, R
-    static constexpr int bD = bA + align_up((int)sizeof(R) * 7 * NLC, 16);  // [NLC][14] dU, R
-    // U = (F, q_proj) staged in FP64 from P1 to P1b; after P1b the same bytes
-    // hold the characteristic fluxes Fs [7][NI] (R, P3 -> P4) and the
-    // interface fluxes dF [7][NI] (FP64, P4 -> P5)
-    static constexpr int bU = bD + align_up((int)sizeof(R) * 14 * NLC, 16);
-    static constexpr int offdF = align_up((int)sizeof(R) * 7 * NI, 8);
-    static constexpr int szU0 = 8 * 14 * NLC;
-    static constexpr int szU1 = offdF + 8 * 7 * NI;
-    // [NS][NI] eigen-system scalars of the interfaces (P2a -> P3, P4): the
-    // left rows and right columns are rebuilt from them in registers where
-    // they are used, never stored
-    static constexpr int bS = bU + align_up(szU0 > szU1 ? szU0 : szU1, 16);
-    static constexpr int bB = bS + align_up((int)sizeof(R) * NS * NI, 16);   // NBUF + NOB mbarriers
-    static constexpr int szB = align_up(8 * (NBUF + NOB), 16);
-    // routing (MODE 1-3): decision, compacted list, weight deviation and FP32
-    // features of the tile's interfaces (collection), the linear flux's LF
-    // speed, the cells' routing values (guard and collection)
-    static constexpr int bDec = bB + szB;                         // [NLF] int
-    static constexpr int bList = bDec + align_up(4 * NLF, 16);    // [NLF] int
-    static constexpr int bDev = bList + align_up(4 * NLF, 16);    // [NLF] float (bits)
-    static constexpr int bFlx = bDev + align_up(4 * NLF, 16);     // [NLF] float (bits): flux departure
-    static constexpr int bFt = bFlx + align_up(4 * NLF, 16);      // [NLF][6] float
-    static constexpr int bAmx = bFt + align_up(4 * 6 * NLF, 16);  // [NLF] R: linear-flux LF speed
-    static constexpr int bCF = bAmx + align_up((int)sizeof(R) * NLF, 16);   // [5][NLC] float cell features
-    static constexpr int bDecW = bCF + align_up(4 * 5 * NLC, 16);  // [NL][F+2] int: fetched decisions
-    static constexpr int bEnd = bDecW + align_up(4 * NL * (F + 2), 16);
-    // learned routing (MODE 1) keeps only what it uses: decisions, list, LF
-    // speed, the cells' density and pressure (the guard), fetched decisions
-    // (two sets: this tile's and the next tile's)
-    static constexpr int lDec = bB + szB;
-    static constexpr int lList = lDec + align_up(4 * NLF, 16);
-    static constexpr int lAmx = lList + align_up(4 * NLF, 16);
-    static constexpr int lCF = lAmx + align_up((int)sizeof(R) * NLF, 16);
-    static constexpr int lDecW = lCF + align_up(4 * 2 * NLC, 16);
-    static constexpr int lEnd = lDecW + 2 * align_up(4 * NL * (F + 2), 16);
-    static constexpr size_t bytes_learned = (size_t)lEnd;
-    static constexpr size_t bytes_plain = (size_t)bB + (NBUF + NOB) * 8;
-    static constexpr size_t bytes_route = (size_t)bEnd;
-    static constexpr uint32_t in_bytes = 8u * NQ;
-    static constexpr uint32_t out_bytes = 8u * NO;
+// One warp's shared memory.  Window arrays are [row][column], a column per
+// (cell, line) with the lines fastest: the first H cells are the last of the
+// chunk before, the other 32 columns are the lanes' new cells.  Consecutive
+// lanes read consecutive columns at every stencil offset, so no access has a
+// bank conflict, and the offset is an immediate.
+template <int DIR, int NL, typename R, int MODE>
+struct WarpMem {
+    static constexpr int W = 32 / NL;                 // cells (and interfaces) per line and chunk
+    // the x sweep's operand tile starts one cell early: its innermost TMA
+    // coordinate has to be even, and the raw tile's start fb+5 is
+    static constexpr int TO = DIR == 0 ? W + 2 : W;
+    // cells of history: differences 4, |lambda| 5, primitives and fluxes 3,
+    // and 4 for the three primitives the four-point CT average reads
+    static constexpr int HD = 4, HL = 5, HP = 3, HB = 4;
+    static constexpr int CD = HD * NL + 32, CL = HL * NL + 32, CP = HP * NL + 32, CB = HB * NL + 32;
+    static constexpr int NCF = MODE == 3 ? 5 : MODE != 0 ? 2 : 0;   // routing values per cell, FP32
+    static constexpr int bRaw = 0;                                  // [8][...] raw conserved of the new cells
+    static constexpr int bOp = bRaw + 8 * 8 * 32;                   // [8][...] update operand
+    static constexpr int bP = align_up(bOp + 8 * 8 * NL * TO, 128); // [5][CP] rho vx By Bz H
+    static constexpr int bF = bP + 8 * 5 * CP;                      // [7][CP] cell fluxes
+    static constexpr int bB = align_up(bF + 8 * 7 * CP, 16);        // [3][CB] vy vz Bx
+    static constexpr int bU = bB + 8 * 3 * CB;                      // [4][NL] M, E of the last cell before
+    static constexpr int bX = bU + 8 * 4 * NL;                      // [7][NL] interface flux before
+    static constexpr int bBar = bX + 8 * 7 * NL;                    // 2 mbarriers: raw, operand
+    static constexpr int bD = align_up(bBar + 16, 16);              // [14][CD] differences of (F, q), R
+    static constexpr int bL = align_up(bD + (int)sizeof(R) * 14 * CD, 16);   // [7][CL] |lambda|, R
+    static constexpr int bC = align_up(bL + (int)sizeof(R) * 7 * CL, 16);    // [NCF][CL] FP32
+    static constexpr int bytes = align_up(bC + 4 * NCF * CL, 128);
+    static constexpr uint32_t raw_bytes = 8u * 8 * 32;
+    static constexpr uint32_t op_bytes = 8u * 8 * NL * TO;
+    static_assert(HL * NL <= 32, "the window shift moves at most one column per lane");
 };
 
-enum { S_VX, S_VY, S_VZ, S_BY, S_BZ, S_VV2, S_CS, S_CS2, S_LF, S_LS, S_AF, S_AS, S_BTY,
-       S_BTZ, S_SGNBX, S_SQR, S_ISQR, S_SGNBT, S_FLIP, S_BTV, S_ICS2 };
+// The move of a window array's last COLS columns to its front, in two steps so
+// that a warp issues every load before the first store (the compiler cannot
+// rule out that they alias): 16-byte moves where the rows allow it, a power of
+// two of lanes per row.
+template <typename T, int ROWS, int PITCH, int COLS>
+struct MoveBack {
+    static constexpr bool VEC = PITCH * sizeof(T) % 16 == 0 && COLS * sizeof(T) % 16 == 0;
+    static constexpr int E = VEC ? 16 / (int)sizeof(T) : 1;
+    static constexpr int per_row(int n) { int p = 1; while (p < n) p *= 2; return p; }
+    static constexpr int PER = per_row(COLS / E), RPI = 32 / PER, N = (ROWS + RPI - 1) / RPI;
+    using V = std::conditional_t<VEC, float4, T>;
+    V v[N];
+    static __device__ __forceinline__ bool mine(int i, int lane) {
+        return i * RPI + lane / PER < ROWS && lane % PER < COLS / E;
+    }
+    // s: the array's first row and column
+    __device__ __forceinline__ void load(const T* s, int lane) {
+        const T* at = s + lane / PER * PITCH + lane % PER * E + 32;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (mine(i, lane)) v[i] = *reinterpret_cast<const V*>(at + i * RPI * PITCH);
+    }
+    __device__ __forceinline__ void store(T* s, int lane) const {
+        T* at = s + lane / PER * PITCH + lane % PER * E;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (mine(i, lane)) *reinterpret_cast<V*>(at + i * RPI * PITCH) = v[i];
+    }
+};
+
+// One half of the WENO5-JS split (src/ssprk.cpp:883-937) from its four
+// arguments (twice the LLF-split differences; see weno_flux).  A common
+// factor of the three indicators cancels from the weights, so they are scaled
+// by 1/3 and eps with them: IS_k / 3 = 13/3 t^2 + t'^2.
+//   w0 = P / D, w2 = 3 Q / D with e_k = (eps + IS_k)^2, P = e1 e2, Q = e0 e1,
+//   D = P + 6 e0 e2 + 3 Q;  X0, X1: the two second differences.
+template <typename R>
+struct WenoHalf { R e0, e1, e2, X0, X1; };
 
 template <typename R>
-__device__ __forceinline__ R sign1(R x) { return (x >= R(0)) ? R(1) : R(-1); }
-
-// The eigenvectors at one interface (src/ssprk.cpp:662-818), rebuilt from its
-// eigen-system scalars S[k * NI] (the S_* table above) where they are used.
-// Column / row m = 0..6 is the field with eigenvalue v - c_f, v - c_a,
-// v - c_s, v, v + c_s, v + c_a, v + c_f.
-//
-// The four magnetosonic fields share one form: with sigma = -1 (m = 0, 2) or
-// +1 (m = 4, 6), and for the fast fields (m = 0, 6) (a1, a2, l1, l2, tau) =
-// (alpha_f, alpha_s, c_f, c_s, +1), for the slow ones (m = 2, 4)
-// (alpha_s, alpha_f, c_s, c_f, -1), the reference's four row (and column)
-// formulas are one expression in those symbols, so the seven lanes that
-// build the seven rows of an interface take three branches, not seven.
-//
-// Sign convention (src/ssprk.cpp:789-818): the fast columns (m = 0, 6), or
-// the slow ones (m = 2, 4) when c_s >= c_a, change sign with sgn(B_t).
-template <typename R, int NI>
-__device__ __forceinline__ R eig_col_sign(int m, const R* S) {
-    const bool flip24 = S[S_FLIP * NI] != R(0);
-    const bool flip = flip24 ? (m == 2 || m == 4) : (m == 0 || m == 6);
-    return flip ? S[S_SGNBT * NI] : R(1);
-}
-
-// Left-eigenvector row m, normalised (src/ssprk.cpp:662-726).
-template <typename R, int NI>
-__device__ __forceinline__ void eig_left_row(int m, const R* S, R gam0, R gam1, R* L) {
-    if (m == 3) {
-        // row (-c^2/gam0 - v^2/2, v, B_t, -1) times s = -gam0/c^2; its first
-        // entry (-c^2/gam0 - v^2/2) s = 1 - (v^2/2) s needs no division
-        const R ics2 = S[S_ICS2 * NI], vv2 = S[S_VV2 * NI];
-        const R s = -gam0 * ics2;
-        L[0] = R(1) - R(0.5) * vv2 * s;
-        L[1] = S[S_VX * NI] * s; L[2] = S[S_VY * NI] * s; L[3] = S[S_VZ * NI] * s;
-        L[4] = S[S_BY * NI] * s; L[5] = S[S_BZ * NI] * s; L[6] = -s;
-    } else if (m == 1 || m == 5) {
-        const R rs = m == 1 ? R(-1) : R(1);
-        const R bty = S[S_BTY * NI], btz = S[S_BTZ * NI], sb = S[S_SGNBX * NI] * S[S_SQR * NI];
-        L[0] = R(0.5) * (btz * S[S_VY * NI] - bty * S[S_VZ * NI]);
-        L[1] = R(0); L[2] = R(-0.5) * btz; L[3] = R(0.5) * bty;
-        L[4] = R(0.5) * (rs * btz * sb); L[5] = R(0.5) * (-rs * bty * sb); L[6] = R(0);
-    } else {
-        const bool fast = m == 0 || m == 6;
-        const R sig = m < 3 ? R(-1) : R(1), tau = fast ? R(1) : R(-1), ts = tau * sig;
-        const R af = S[S_AF * NI], as = S[S_AS * NI], lf = S[S_LF * NI], ls = S[S_LS * NI];
-        const R a1 = fast ? af : as, a2 = fast ? as : af, l1 = fast ? lf : ls, l2 = fast ? ls : lf;
-        const R vx = S[S_VX * NI], sgnBx = S[S_SGNBX * NI], bty = S[S_BTY * NI], btz = S[S_BTZ * NI];
-        const R a2l2 = ts * a2 * l2 * sgnBx, csa2 = tau * S[S_CS * NI] * a2 * S[S_SQR * NI];
-        L[0] = a1 * (gam1 * S[S_VV2 * NI] - sig * l1 * vx) + a2l2 * S[S_BTV * NI];
-        L[1] = a1 * (gam0 * vx + sig * l1);
-        L[2] = gam0 * a1 * S[S_VY * NI] - a2l2 * bty;
-        L[3] = gam0 * a1 * S[S_VZ * NI] - a2l2 * btz;
-        L[4] = gam0 * a1 * S[S_BY * NI] + csa2 * bty;
-        L[5] = gam0 * a1 * S[S_BZ * NI] + csa2 * btz;
-        L[6] = -gam0 * a1;
-        // normalisation and the sign convention (only magnetosonic rows flip)
-        const R s = R(0.5) * S[S_ICS2 * NI] * eig_col_sign<R, NI>(m, S);
-#pragma unroll
-        for (int k = 0; k < 7; ++k) L[k] *= s;
-    }
-}
-
-// Row r of the right-eigenvector matrix, R(r, m) for m = 0..6
-// (src/ssprk.cpp:729-787): component r of every column.
-template <typename R, int NI>
-__device__ __forceinline__ void eig_right_row(int r, const R* S, R gam2, R* Rr) {
-    const R af = S[S_AF * NI], as = S[S_AS * NI];
-    switch (r) {
-        case 0:
-            Rr[0] = af; Rr[1] = R(0); Rr[2] = as; Rr[3] = R(1); Rr[4] = as; Rr[5] = R(0); Rr[6] = af;
-            break;
-        case 1: {
-            const R vx = S[S_VX * NI], lf = S[S_LF * NI], ls = S[S_LS * NI];
-            Rr[0] = af * (vx - lf); Rr[1] = R(0); Rr[2] = as * (vx - ls); Rr[3] = vx;
-            Rr[4] = as * (vx + ls); Rr[5] = R(0); Rr[6] = af * (vx + lf);
-            break;
-        }
-        case 2:
-        case 3: {
-            const R v = S[(r == 2 ? S_VY : S_VZ) * NI], bt = S[(r == 2 ? S_BTY : S_BTZ) * NI];
-            const R sgnBx = S[S_SGNBX * NI];
-            const R pf = as * S[S_LS * NI] * bt * sgnBx, ps = af * S[S_LF * NI] * bt * sgnBx;
-            const R alf = r == 2 ? -S[S_BTZ * NI] : S[S_BTY * NI];
-            Rr[0] = af * v + pf; Rr[1] = alf; Rr[2] = as * v - ps; Rr[3] = v;
-            Rr[4] = as * v + ps; Rr[5] = alf; Rr[6] = af * v - pf;
-            break;
-        }
-        case 4:
-        case 5: {
-            const R bt = S[(r == 4 ? S_BTY : S_BTZ) * NI], isqr = S[S_ISQR * NI];
-            const R cs = S[S_CS * NI];
-            const R f = cs * as * bt * isqr, sl = -cs * af * bt * isqr;
-            const R alf = (r == 4 ? -S[S_BTZ * NI] : S[S_BTY * NI]) * S[S_SGNBX * NI] * isqr;
-            Rr[0] = f; Rr[1] = alf; Rr[2] = sl; Rr[3] = R(0); Rr[4] = sl; Rr[5] = -alf; Rr[6] = f;
-            break;
-        }
-        default: {
-            const R vx = S[S_VX * NI], vv2 = S[S_VV2 * NI], lf = S[S_LF * NI], ls = S[S_LS * NI];
-            const R h = R(0.5) * vv2 - gam2 * S[S_CS2 * NI];
-            const R btv = S[S_BTV * NI] * S[S_SGNBX * NI];
-            const R pf = as * ls * btv, ps = af * lf * btv;
-            const R alf = S[S_BTY * NI] * S[S_VZ * NI] - S[S_BTZ * NI] * S[S_VY * NI];
-            Rr[0] = af * (lf * lf - lf * vx + h) + pf; Rr[1] = alf;
-            Rr[2] = as * (ls * ls - ls * vx + h) - ps; Rr[3] = R(0.5) * vv2;
-            Rr[4] = as * (ls * ls + ls * vx + h) + ps; Rr[5] = alf;
-            Rr[6] = af * (lf * lf + lf * vx + h) - pf;
-            break;
-        }
-    }
-    const R sgnBt = S[S_SGNBT * NI];
-    if (S[S_FLIP * NI] != R(0)) { Rr[2] *= sgnBt; Rr[4] *= sgnBt; }
-    else { Rr[0] *= sgnBt; Rr[6] *= sgnBt; }
+__device__ __forceinline__ WenoHalf<R> weno_half(R a, R b, R c, R d) {
+    const R K = R(13.0 / 3.0), eps = R(4.0e-10 / 3.0);
+    const R t0 = a - b, t2 = b - c, t4 = c - d;
+    const R t1 = fm(R(-3), b, a), t3 = b + c, t5 = fm(R(3), c, -d);
+    const R d0 = fm(t1, t1, fm(K * t0, t0, eps));
+    const R d1 = fm(t3, t3, fm(K * t2, t2, eps));
+    const R d2 = fm(t5, t5, fm(K * t4, t4, eps));
+    return WenoHalf<R>{d0 * d0, d1 * d1, d2 * d2, t0 - t2, t2 - t4};
 }
 
 // Characteristic WENO5-JS/LLF flux of one field (src/ssprk.cpp:883-937) from
-// the projected cell differences dF_k = L.(F_{k+1} - F_k), dq_k = L.(q_{k+1} - q_k),
-// k = 0..4 over the 6-cell stencil.
+// the projected cell differences f_k = L.(F_{k+1} - F_k), q_k = L.(q_{k+1} - q_k),
+// k = 0..4 over the 6-cell stencil, and the stencil's largest |lambda|.
 //
 // Restated, not transcribed:
 //  * the fourth-order central part (-F1 + 7F2 + 7F3 - F4)/12 equals
-//    F2 + (dF1 + 6 dF2 - dF3)/12; its F2 share is added back in physical
+//    F2 + (f1 + 6 f2 - f3)/12; its F2 share is added back in physical
 //    space after the back-projection (R L = I), so only the correction is
 //    returned;
-//  * the LLF-split arguments 0.5 (dF +- amx dq) are used without the 0.5:
+//  * the LLF-split arguments 0.5 (f +- amx q) are used without the 0.5:
 //    doubling a, b, c, d quadruples every smoothness indicator, so with
 //    eps -> 4 eps the nonlinear weights are unchanged and the 0.5 moves onto
 //    the linear combination (1/3 -> 1/6, 1/6 -> 1/12);
-//  * FP64: omega0 = a0 / (a0 + a1 + a2) with a_k = c_k / (eps + IS_k)^2 is
-//    e1 e2 / D with e_k = (eps + IS_k)^2 and D = e1 e2 + 6 e0 e2 + 3 e0 e1
-//    (omega2 = 3 e0 e1 / D); the two halves share one division 1/(D+ D-).
-//    FP32 keeps the a_k form (the products of e_k would underflow) with fast
-//    reciprocals.
-template <typename R>
-__device__ __forceinline__ R weno_half_w(R a, R b, R c, R d, R& w0, R& w2) {
-    const R eps4 = R(4.0e-10);
-    const R t0 = a - b, t1 = a - R(3) * b;
-    const R t2 = b - c, t3 = b + c;
-    const R t4 = c - d, t5 = R(3) * c - d;
-    const R d0 = eps4 + (R(13) * t0 * t0 + R(3) * t1 * t1);
-    const R d1 = eps4 + (R(13) * t2 * t2 + R(3) * t3 * t3);
-    const R d2 = eps4 + (R(13) * t4 * t4 + R(3) * t5 * t5);
-    if constexpr (std::is_same<R, double>::value) {
-        const R e0 = d0 * d0, e1 = d1 * d1, e2 = d2 * d2;
-        w0 = e1 * e2;                       // numerators; the caller divides by D
-        w2 = R(3) * (e0 * e1);
-        return w0 + R(6) * (e0 * e2) + w2;  // D
-    } else {
-        const R a0 = Math<R>::rcp(d0 * d0);
-        const R a1 = R(6) * Math<R>::rcp(d1 * d1);
-        const R a2 = R(3) * Math<R>::rcp(d2 * d2);
-        const R is = Math<R>::rcp(a0 + a1 + a2);
-        w0 = a0 * is;
-        w2 = a2 * is;
-        return R(1);
-    }
-}
-
-template <typename R, bool DEV = false>
-__device__ __forceinline__ R weno_flux_d(const R* dF, const R* dq, R amx, R* dev = nullptr) {
-    const R ap = dF[0] + amx * dq[0], bp = dF[1] + amx * dq[1], cp = dF[2] + amx * dq[2], dp = dF[3] + amx * dq[3];
-    const R am = dF[4] - amx * dq[4], bm = dF[3] - amx * dq[3], cm = dF[2] - amx * dq[2], dm = dF[1] - amx * dq[1];
-    R w0p, w2p, w0m, w2m;
-    const R Dp = weno_half_w(ap, bp, cp, dp, w0p, w2p);
-    const R Dm = weno_half_w(am, bm, cm, dm, w0m, w2m);
-    if constexpr (std::is_same<R, double>::value) {
-        double ip, im;
-        const double DD = Dp * Dm;
-        if (DD < 1.0e300) { const double r = 1.0 / DD; ip = Dm * r; im = Dp * r; }
-        else { ip = 1.0 / Dp; im = 1.0 / Dm; }
-        w0p *= ip; w2p *= ip; w0m *= im; w2m *= im;
-    }
+//  * FP64: a half's weighted second differences are w / 6 - X1 / 24 with
+//    w = (P / D) X0 + 1.5 (Q / D) X1.  FP32 keeps the weights c_k / e_k (the
+//    products of e_k would underflow) with fast reciprocals.
+template <bool DEV>
+__device__ __forceinline__ double weno_flux(const double* f, const double* q, double amx, double* dev) {
+    const WenoHalf<double> p = weno_half(fm(amx, q[0], f[0]), fm(amx, q[1], f[1]), fm(amx, q[2], f[2]),
+                                         fm(amx, q[3], f[3]));
+    const WenoHalf<double> m = weno_half(fm(-amx, q[4], f[4]), fm(-amx, q[3], f[3]), fm(-amx, q[2], f[2]),
+                                         fm(-amx, q[1], f[1]));
+    const double Pp = p.e1 * p.e2, Qp = p.e0 * p.e1, Dp = fm(6.0, p.e0 * p.e2, fm(3.0, Qp, Pp));
+    const double Pm = m.e1 * m.e2, Qm = m.e0 * m.e1, Dm = fm(6.0, m.e0 * m.e2, fm(3.0, Qm, Pm));
+    // (the weights before their products with X: P X would overflow first)
+    const double ip = near_recip(Dp), im = near_recip(Dm);
+    const double wp = fm(1.5, (Qp * ip) * p.X1, (Pp * ip) * p.X0), wm = fm(1.5, (Qm * im) * m.X1, (Pm * im) * m.X0);
     if constexpr (DEV) {
         // largest departure of the nonlinear weights from the linear (0.1, 0.6, 0.3)
-        const R w1p = R(1) - w0p - w2p, w1m = R(1) - w0m - w2m;
-        R d = fabs(w0p - R(0.1));
-        d = fmax(d, fabs(w1p - R(0.6))); d = fmax(d, fabs(w2p - R(0.3)));
-        d = fmax(d, fabs(w0m - R(0.1))); d = fmax(d, fabs(w1m - R(0.6))); d = fmax(d, fabs(w2m - R(0.3)));
-        *dev = d;
+        const double w0p = Pp / Dp, w2p = 3.0 * Qp / Dp, w0m = Pm / Dm, w2m = 3.0 * Qm / Dm;
+        double d = fmax(fabs(w0p - 0.1), fabs(w2p - 0.3));
+        d = fmax(d, fabs(1.0 - w0p - w2p - 0.6));
+        d = fmax(d, fmax(fabs(w0m - 0.1), fabs(w2m - 0.3)));
+        *dev = fmax(d, fabs(1.0 - w0m - w2m - 0.6));
     }
-    const R first = (dF[1] + R(6) * dF[2] - dF[3]) * R(1.0 / 12.0);
-    const R second = w0p * (ap - R(2) * bp + cp) * R(1.0 / 6.0) + (w2p - R(0.5)) * (bp - R(2) * cp + dp) * R(1.0 / 12.0);
-    const R third = w0m * (am - R(2) * bm + cm) * R(1.0 / 6.0) + (w2m - R(0.5)) * (bm - R(2) * cm + dm) * R(1.0 / 12.0);
-    return first - second + third;
+    const double c = fm(6.0, f[2], f[1]) - f[3];
+    return fm(1.0 / 6.0, wm - wp, fm(1.0 / 12.0, c, (1.0 / 24.0) * (p.X1 - m.X1)));
+}
+
+template <bool DEV>
+__device__ __forceinline__ float weno_flux(const float* f, const float* q, float amx, float*) {
+    static_assert(!DEV, "labels are recorded by the FP64 method");
+    const WenoHalf<float> p = weno_half(fm(amx, q[0], f[0]), fm(amx, q[1], f[1]), fm(amx, q[2], f[2]),
+                                        fm(amx, q[3], f[3]));
+    const WenoHalf<float> m = weno_half(fm(-amx, q[4], f[4]), fm(-amx, q[3], f[3]), fm(-amx, q[2], f[2]),
+                                        fm(-amx, q[1], f[1]));
+    auto part = [](const WenoHalf<float>& h) {
+        const float a0 = near_recip(h.e0), a1 = 6.0f * near_recip(h.e1), a2 = 3.0f * near_recip(h.e2);
+        const float is = near_recip(a0 + a1 + a2);
+        return fm((a0 * is) * h.X0, 2.0f, fm(a2, is, -0.5f) * h.X1);
+    };
+    const float c = fm(6.0f, f[2], f[1]) - f[3];
+    return (1.0f / 12.0f) * (c - part(p) + part(m));
 }
 
 // Component-wise fifth-order upwind flux with the linear weights
 // (0.1, 0.6, 0.3) and the stencil's largest |lambda| as Lax-Friedrichs speed:
-// the cheap flux a router sends smooth interfaces to.  dF_k, dq_k are the physical cell
-// differences of one component over the stencil; returns the correction to
-// the central F_i (same form as weno_flux_d, no characteristic projection).
+// the cheap flux a router sends smooth interfaces to.  f_k, q_k are the
+// physical cell differences of one component over the stencil; returns the
+// correction to the central F_i (the same form as weno_flux with constant
+// weights, whose second differences then add up to one fifth-order stencil).
 template <typename R>
-__device__ __forceinline__ R linear_flux_d(const R* dF, const R* dq, R amx) {
-    const R ap = dF[0] + amx * dq[0], bp = dF[1] + amx * dq[1], cp = dF[2] + amx * dq[2], dp = dF[3] + amx * dq[3];
-    const R am = dF[4] - amx * dq[4], bm = dF[3] - amx * dq[3], cm = dF[2] - amx * dq[2], dm = dF[1] - amx * dq[1];
-    const R first = (dF[1] + R(6) * dF[2] - dF[3]) * R(1.0 / 12.0);
-    const R second = R(0.1) * (ap - R(2) * bp + cp) * R(1.0 / 6.0) + R(-0.2) * (bp - R(2) * cp + dp) * R(1.0 / 12.0);
-    const R third = R(0.1) * (am - R(2) * bm + cm) * R(1.0 / 6.0) + R(-0.2) * (bm - R(2) * cm + dm) * R(1.0 / 12.0);
-    return first - second + third;
+__device__ __forceinline__ R linear_flux(const R* f, const R* q, R amx) {
+    const R cf = fm(R(7), f[1] - f[3], fm(R(30), f[2], f[4] - f[0]));
+    const R cq = fm(R(6), q[2], fm(R(-4), q[1] + q[3], q[0] + q[4]));
+    return fm(-amx, cq, cf) * R(1.0 / 60.0);
 }
 
 __device__ __forceinline__ constexpr int perm_of(int dir, int v) {
@@ -350,836 +290,698 @@ __device__ __forceinline__ constexpr int perm_of(int dir, int v) {
                     : (v == 1 ? 3 : v == 2 ? 1 : v == 3 ? 2 : v == 4 ? 6 : v == 5 ? 4 : v == 6 ? 5 : v);
 }
 
+// the inverse: the line variable of a conserved index (the y and z
+// permutations are each other's inverses)
+__device__ __forceinline__ constexpr int line_var(int dir, int gv) { return perm_of(dir == 0 ? 0 : 3 - dir, gv); }
+
+// A cell: primit (src/ssprk.cpp:479-512) with v from the unfloored density and
+// floors on rho and p with E recomputed; eigenst centre fluxes (561-593) with
+// the floored values; the eigenvalues in the working type R: FP64 for the plain
+// method, FP32 in the mixed one (where they feed only the FP32 characteristic
+// part).  Primitives and speeds are formed in the reference's own operations
+// and order: where the transverse field vanishes, sqrt(lf^2 - c^2) turns their
+// last bit into 1e-8.
+template <typename R>
+struct CellValues {
+    double rho, vx, vy, vz, EE, HH, F[7];
+    R lam[7];      // |lambda_m|: every reader takes the magnitude (the LLF speeds)
+    float cf[5];   // the routing features' values (MODE 1-3)
+};
+
+template <int MODE, typename R>
+__device__ __forceinline__ void cell_values(const double* q, double gam, double rhomin, double pgmin, CellValues<R>& o) {
+    const double Mx = q[1], My = q[2], Mz = q[3], Bx = q[4], By = q[5], Bz = q[6], gm1 = gam - 1.0;
+    double rho = q[0], EE = q[7];
+    double irho = recip(rho);
+    const double vx = quot(Mx, rho, irho), vy = quot(My, rho, irho), vz = quot(Mz, rho, irho);
+    const double vv2 = vx * vx + vy * vy + vz * vz;
+    const double BB2 = Bx * Bx + By * By + Bz * Bz;
+    double pg = gm1 * (EE - 0.5 * (rho * vv2 + BB2));
+    const bool low = rho < rhomin || pg < pgmin;
+    if (low) {
+        rho = fmax(rhomin, rho);
+        pg = fmax(pgmin, pg);
+        EE = quot(pg, gm1, recip(gm1)) + 0.5 * (rho * vv2 + BB2);
+        irho = recip(rho);
+    }
+    o.rho = rho; o.vx = vx; o.vy = vy; o.vz = vz; o.EE = EE;
+    o.HH = quot(EE + pg, rho, irho);
+    const double pt = fm(0.5, BB2, pg);
+    const double vdB = fm(vz, Bz, fm(vy, By, vx * Bx));
+    o.F[0] = rho * vx;                 // DD (floored) * vx
+    o.F[1] = fm(Mx, vx, fm(-Bx, Bx, pt));
+    o.F[2] = fm(My, vx, -(Bx * By));
+    o.F[3] = fm(Mz, vx, -(Bx * Bz));
+    o.F[4] = fm(By, vx, -(Bx * vy));
+    o.F[5] = fm(Bz, vx, -(Bx * vz));
+    o.F[6] = fm(EE + pt, vx, -(Bx * vdB));
+    R bbn2, bnx2, cs2;
+    if constexpr (std::is_same<R, double>::value) {
+        bbn2 = quot(BB2, rho, irho);
+        bnx2 = quot(Bx * Bx, rho, irho);
+        cs2 = gam * fabs(quot(pg, rho, irho));
+    } else {
+        const R irR = R(irho);
+        bbn2 = R(BB2) * irR;
+        bnx2 = R(Bx * Bx) * irR;
+        cs2 = R(gam) * fabs(R(pg) * irR);
+    }
+    const R bc = bbn2 + cs2;
+    const R rt = root(bc * bc - R(4) * bnx2 * cs2);
+    const R lf = root(R(0.5) * (bc + rt));
+    const R la = root(bnx2);
+    const R ls = root(R(0.5) * (bc - rt));
+    const R vxR = R(vx);
+    o.lam[0] = fabs(vxR - lf); o.lam[1] = fabs(vxR - la); o.lam[2] = fabs(vxR - ls); o.lam[3] = fabs(vxR);
+    o.lam[4] = fabs(vxR + ls); o.lam[5] = fabs(vxR + la); o.lam[6] = fabs(vxR + lf);
+    if constexpr (MODE != 0) {
+        // (the guard needs density and pressure only)
+        o.cf[0] = (float)rho; o.cf[1] = (float)pg;
+        if constexpr (MODE == 3) { o.cf[2] = sqrtf((float)BB2); o.cf[3] = sqrtf((float)vv2); o.cf[4] = (float)lf; }
+    }
+}
+
+// The interface between the first two cells of the window at P (the lane's
+// column): eigen-system, projection, WENO5 of the seven fields and
+// back-projection.  out: the upwind correction to the left cell's flux.
+// before_back runs before the back-projection.
+template <typename R>
+struct FaceValues {
+    R out[7];
+    R rho, hvv, bbn2;    // of the mean state (label collection)
+    float departure;     // largest departure of the nonlinear weights (label collection)
+};
+
+template <int NL, int CP, int CB, int CD, int CL, int MODE, typename R, typename Before>
+__device__ __forceinline__ void face_values(const double* sP, const double* sB, const R* sD, const R* sL, R gamR, R gam2,
+                                            FaceValues<R>& o, Before before_back) {
+    if constexpr (MODE == 3) o.departure = 0.0f;
+    const R gam0 = R(1) - gamR;
+    // eigen-system of the arithmetic mean of the two cells'
+    // primitives (src/ssprk.cpp:610-660)
+    auto mean = [&](const double* s) { return R(0.5 * (s[0] + s[NL])); };
+    const R rho = mean(sP), vx = mean(sP + CP), By = mean(sP + 2 * CP), Bz = mean(sP + 3 * CP);
+    const R HH = mean(sP + 4 * CP);
+    const R vy = mean(sB + NL), vz = mean(sB + CB + NL), Bx = mean(sB + 2 * CB + NL);
+    const R vv2 = vx * vx + vy * vy + vz * vz;
+    const R BB2 = Bx * Bx + By * By + Bz * Bz;
+    R bbn2, bnx2;
+    const R isqr = root_inverse(rho);
+    if constexpr (std::is_same<R, double>::value) {
+        const double irho = recip(rho);
+        bbn2 = quot(BB2, rho, irho);
+        bnx2 = quot(Bx * Bx, rho, irho);
+    } else {
+        const R irho = isqr * isqr;
+        bbn2 = BB2 * irho;
+        bnx2 = Bx * Bx * irho;
+    }
+    const R cs2 = (gamR - R(1)) * (HH - R(0.5) * (vv2 + bbn2));
+    const R cs = root(cs2);
+    const R bc = bbn2 + cs2;
+    const R rt = root(bc * bc - R(4) * bnx2 * cs2);
+    const R lf = root(R(0.5) * (bc + rt));
+    const R ls = root(R(0.5) * (bc - rt));
+    const R Bt2 = By * By + Bz * Bz;
+    const bool some = Bt2 >= R(1.0e-30);
+    const R ib = root_inverse(Bt2), h = R(0.70710678118654752440);
+    const R bty = some ? By * ib : h, btz = some ? Bz * ib : h;
+    const R df = lf * lf - ls * ls;
+    const bool wide = df >= R(1.0e-30);
+    const R idf = root_inverse(df);
+    const R af = wide ? root(cs2 - ls * ls) * idf : R(1), as = wide ? root(lf * lf - cs2) * idf : R(1);
+    const R hvv = R(0.5) * vv2, sqr = rho * isqr;
+    const R ics2 = near_recip(cs2);
+    const R sgnB = (Bx >= R(0)) ? R(1) : R(-1);
+    const R btv = fm(bty, vy, btz * vz);
+
+    // Left eigenvectors (src/ssprk.cpp:662-726) applied to the
+    // stencil's differences.  The four magnetosonic rows are
+    // even +- odd combinations of four products with D that do
+    // not depend on the field,
+    //   e = (-v^2/2, v, B_t, -1).D    b = beta.(D4, D5)
+    //   x = D1 - vx D0                t = beta.(D2, D3) - beta.v D0
+    // with coefficients below for the fast and the slow pair; the
+    // entropy row is D0 + s e, and the two Alfven rows are even
+    // +- odd in (beta x) the transverse momenta and fields.
+    // (The reference turns the fast or slow rows and columns by
+    // sgn(B_t), src/ssprk.cpp:789-818; the field's flux is odd in
+    // its row, so the sign cancels exactly from row and column.)
+    auto field = [&](int m, const R* pf, const R* pq) -> R {
+        const R* sm = sL + m * CL;
+        R amx = sm[0];
+#pragma unroll
+        for (int k = 1; k < 6; ++k) amx = larger(amx, sm[k * NL]);
+        R d = R(0);
+        const R r = weno_flux<MODE == 3>(pf, pq, amx, &d);
+        if constexpr (MODE == 3) o.departure = fmaxf(o.departure, (float)d);
+        return r;
+    };
+    const R hn = R(0.5) * ics2;   // the rows' normalisation
+    const R cen = -gam0 * ics2;
+    // Three pairs of fields, one loop body: fast (0, 6) with the
+    // entropy field, slow (2, 4), Alfven (1, 5).  Unrolled, the
+    // chunk's code no longer fits the instruction caches (0.5 ms
+    // of 3.8 per 256^3 sweep); and the differences are read once
+    // per pair, since two pairs' products do not fit 168 registers.
+    R F0, F1, F2, F3, F4, F5, F6;
+#pragma unroll 1
+    for (int pair = 0; pair < 3; ++pair) {
+        R mn[2][5], pl[2][5];
+        if (pair < 2) {
+            const bool slow_pair = pair == 1;
+            const R a1 = slow_pair ? as : af, a2 = slow_pair ? af : as, l1 = slow_pair ? ls : lf,
+                    l2 = slow_pair ? lf : ls, tau = slow_pair ? R(-1) : R(1);
+            const R ce = hn * gam0 * a1, cb = tau * hn * cs * a2 * sqr, cx = hn * l1 * a1,
+                    ct = -tau * hn * a2 * l2 * sgnB;
+            R en[2][5];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const R* D = sD + (7 * h) * CD + k * NL;
+                    const R D0 = D[0], D1 = D[CD], D2 = D[2 * CD], D3 = D[3 * CD], D4 = D[4 * CD],
+                            D5 = D[5 * CD];
+                    const R e = fm(-hvv, D0, fm(vx, D1, fm(vy, D2, fm(vz, D3, fm(By, D4, fm(Bz, D5, -D[6 * CD]))))));
+                    const R b = fm(bty, D4, btz * D5);
+                    const R x = fm(-vx, D0, D1);
+                    const R t = fm(bty, D2, fm(btz, D3, -btv * D0));
+                    const R ev = fm(ce, e, cb * b), od = fm(cx, x, ct * t);
+                    mn[h][k] = ev - od;
+                    pl[h][k] = ev + od;
+                    en[h][k] = fm(cen, e, D0);
+                }
+            if (pair == 0) F3 = field(3, en[0], en[1]);
+        } else {
+            const R cv = R(0.5) * fm(btz, vy, -(bty * vz)), cy = R(0.5) * bty, cz = R(0.5) * btz;
+            const R cb = sgnB * sqr, cby = cb * cy, cbz = cb * cz;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const R* D = sD + (7 * h) * CD + k * NL;
+                    const R ev = fm(cv, D[0], fm(cy, D[3 * CD], -(cz * D[2 * CD])));
+                    const R od = fm(cbz, D[4 * CD], -(cby * D[5 * CD]));
+                    mn[h][k] = ev - od;
+                    pl[h][k] = ev + od;
+                }
+        }
+        const int m = pair == 0 ? 0 : 3 - pair;   // 0, 2, 1
+        const R lo = field(m, mn[0], mn[1]), hi = field(6 - m, pl[0], pl[1]);
+        if (pair == 0) { F0 = lo; F6 = hi; }
+        else if (pair == 1) { F2 = lo; F4 = hi; }
+        else { F1 = lo; F5 = hi; }
+    }
+
+    before_back();
+    // Right eigenvectors (src/ssprk.cpp:729-787) by the same
+    // symmetry: sums and differences of the paired fields
+    const R fs = af * (F0 + F6), ss = as * (F2 + F4);
+    const R fd = af * lf * (F6 - F0), sd = as * ls * (F4 - F2);
+    const R w = sgnB * fm(as * ls, F0 - F6, (af * lf) * (F4 - F2));
+    const R u = F1 + F5, du = sgnB * isqr * (F1 - F5);
+    const R bq = cs * isqr * fm(as, F0 + F6, -af * (F2 + F4));
+    R* out = o.out;
+    out[0] = fs + ss + F3;
+    out[1] = fm(vx, out[0], fd + sd);
+    out[2] = fm(vy, out[0], fm(bty, w, -(btz * u)));
+    out[3] = fm(vz, out[0], fm(btz, w, bty * u));
+    out[4] = fm(bty, bq, -(btz * du));
+    out[5] = fm(btz, bq, bty * du);
+    const R gc = gam2 * cs2;
+    out[6] = fm(hvv, out[0], fm(lf * lf - gc, fs, fm(ls * ls - gc, ss, fm(vx, fd + sd,
+                fm(btv, w, fm(bty, vz, -(btz * vy)) * u)))));
+    if constexpr (MODE == 3) { o.rho = rho; o.hvv = hvv; o.bbn2 = bbn2; }
+}
+
 constexpr uint32_t kWaitLimit = 1u << 26;   // bounded TMA wait (~seconds), then flag and skip
+
+// How a direction's lines are cut into work items (one warp each).  Lines of
+// the x sweep start at j = 3; lines of the y/z sweeps are NL consecutive i
+// from a multiple of NL (masked ghost lines at the ends), so that a tile row
+// is a whole 32-byte sector for NL = 4 and the innermost TMA coordinate is
+// even.  A segment of `chunks` chunks advances chunks * W - ov cells: its
+// first interface repeats the segment before's last (ov = 1; in x ov = 2 and
+// the first interface is -1, which keeps the raw tiles' x even).
+template <int DIR, int NL>
+struct Cut {
+    static constexpr int W = 32 / NL, ov = DIR == 0 ? 2 : 1, f0 = DIR == 0 ? -1 : 0, line0 = DIR == 0 ? 3 : 0;
+    int n, nt1, nt2, groups, segs;
+    __host__ __device__ Cut(const Grid& g, int chunks) {
+        n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
+        nt1 = DIR == 0 ? g.ny : g.nx;
+        nt2 = DIR == 2 ? g.ny : g.nz;
+        groups = (3 + nt1 - line0 + NL - 1) / NL;
+        const int step = chunks * W - ov;
+        segs = (n + step - 1) / step;
+    }
+    __host__ __device__ long long items() const { return (long long)groups * segs * nt2; }
+};
 
 // MODE 0: plain method.  1: learned routing (network + guard).  2: guard-only
 // routing (the ablation).  3: plain method that also records features and
 // nonlinear-weight labels of sampled tiles for training.
 //
 // ENS: one launch advances this sweep for every member of a batched
-// ensemble; the global tile index runs over the members' tiles in order, and
-// each tile reads its member's arguments from the ensemble table.
-template <int DIR, int NL, int T, int NT, typename R, int MINB, int MODE, bool ENS = false>
-__global__ void __launch_bounds__(NT, MINB) k_sweep(const __grid_constant__ SweepArgs a0) {
+// ensemble; the global item index runs over the members' items in order, and
+// each item reads its member's arguments from the ensemble table.
+template <int DIR, int NL, int WPB, typename R, int MINB, int MODE, bool ENS = false>
+__global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant__ SweepArgs a0) {
     static_assert(!ENS || MODE == 0, "ensembles run the plain method");
+    static_assert(MODE != 3 || std::is_same<R, double>::value, "labels are recorded by the FP64 method");
     constexpr bool ROUTED = MODE == 1 || MODE == 2;
-    using TL = Tile<DIR, NL, T, R>;
-    using V2 = typename Math<R>::V2;
-    constexpr int C = TL::C, F = TL::F, NP = TL::NP, NLC = TL::NLC, NLF = TL::NLF, NI = TL::NI;
-    constexpr int TO = TL::TO;
-    constexpr int NBUF = TL::NBUF, NOB = TL::NOB;
-    constexpr int FE = F + 2;                                  // fetched decisions per line (MODE 1)
-    constexpr int DWS = align_up(4 * NL * FE, 16) / 4;         // ints per decision set
+    using M = WarpMem<DIR, NL, R, MODE>;
+    using CUT = Cut<DIR, NL>;
+    constexpr int W = M::W, CD = M::CD, CL = M::CL, CP = M::CP, CB = M::CB;
+    constexpr unsigned ALL = 0xffffffffu;
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(ALL, threadIdx.x >> 5, 0);   // (uniform in the warp)
+    const int l = lane % NL, j = lane / NL;   // the lane's line and its place along the chunk
     // TMA destinations need 128-byte alignment: align the carve-up base
-    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-    double* sFc = reinterpret_cast<double*>(sm + TL::bFc);
-    double* sP = reinterpret_cast<double*>(sm + TL::bP);
-    R* sA = reinterpret_cast<R*>(sm + TL::bA);
-    R* sD = reinterpret_cast<R*>(sm + TL::bD);
-    double* sUst = reinterpret_cast<double*>(sm + TL::bU);   // U staging (P1 -> P1b), FP64
-    R* sFs = reinterpret_cast<R*>(sm + TL::bU);                        // [7][NI], P3 -> P4
-    double* sdF = reinterpret_cast<double*>(sm + TL::bU + TL::offdF);   // [7][NI], P4 -> P5
-    R* sS = reinterpret_cast<R*>(sm + TL::bS);                         // [NS][NI], P2a -> P3, P4
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + TL::bB);
-    constexpr bool LM = MODE == 1;   // the learned mode's compact layout
-    int* sDec = reinterpret_cast<int*>(sm + (LM ? TL::lDec : TL::bDec));       // 1: full WENO, 0: linear flux
-    int* sList = reinterpret_cast<int*>(sm + (LM ? TL::lList : TL::bList));    // full-WENO interfaces
-    float* sDev = reinterpret_cast<float*>(sm + TL::bDev);      // weight deviation (collect)
-    float* sFlx = reinterpret_cast<float*>(sm + TL::bFlx);      // flux departure (collect)
-    float* sFt = reinterpret_cast<float*>(sm + TL::bFt);        // features (collect)
-    R* sAmx = reinterpret_cast<R*>(sm + (LM ? TL::lAmx : TL::bAmx));           // per interface: max |lambda_0|, |lambda_6|
-    float* sCF = reinterpret_cast<float*>(sm + (LM ? TL::lCF : TL::bCF));      // per cell: rho, p, |B|, |v|, c_f
-    int* sDecW = reinterpret_cast<int*>(sm + (LM ? TL::lDecW : TL::bDecW));    // MODE 1: fetched decisions
-    __shared__ int s_nfull;
-    __shared__ unsigned int s_cnt[2];   // full, cheap interfaces
+    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127)) +
+                        warp * M::bytes;
+    const double* sRaw = reinterpret_cast<const double*>(sm + M::bRaw);
+    const double* sOp = reinterpret_cast<const double*>(sm + M::bOp);
+    // window arrays, at the lane's column: the cell s places after the first
+    // of the window is s * NL further (a new cell is H * NL further)
+    double* sP = reinterpret_cast<double*>(sm + M::bP) + lane;
+    double* sB = reinterpret_cast<double*>(sm + M::bB) + lane;
+    double* sF = reinterpret_cast<double*>(sm + M::bF) + lane;
+    R* sD = reinterpret_cast<R*>(sm + M::bD) + lane;
+    R* sL = reinterpret_cast<R*>(sm + M::bL) + lane;
+    float* sC = reinterpret_cast<float*>(sm + M::bC) + lane;
+    double* sU = reinterpret_cast<double*>(sm + M::bU) + l;
+    double* sX = reinterpret_cast<double*>(sm + M::bX) + l;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + M::bBar);
 
-    // Tiles: T active cells along the sweep x NL lines x one plane.  Lines of
-    // the x sweep start at j = 3; lines of the y/z sweeps are consecutive i and
-    // start at the even i = 2 (a masked ghost line) so the innermost TMA
-    // coordinate stays 16-byte aligned.
-    struct Geo { int n, nt1, ntx, nty; long long sstride; };
-    auto geo_of = [](const Grid& g) -> Geo {
-        Geo o;
-        o.n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
-        o.nt1 = DIR == 0 ? g.ny : g.nx;
-        o.sstride = DIR == 0 ? 1ll : DIR == 1 ? (long long)g.pitch : (long long)g.pitch * g.P1;
-        o.ntx = (o.n + T - 1) / T;
-        o.nty = DIR == 0 ? (o.nt1 + NL - 1) / NL : (o.nt1 + 1 + NL - 1) / NL;
-        return o;
-    };
-    const int line0 = DIR == 0 ? 3 : 2;
-    // global tile -> member (ENS) and the member's arguments + local tile
-    auto member_of = [&](long long tile) -> int {
-        int lo = 0, hi = a0.ens_n - 1;   // last member whose first tile is <= tile
+    // one place of the march: an item's segment and the chunk in it (-1: the
+    // five cells before the first interface, no interface yet)
+    struct Place { long long item; const SweepArgs* a; int t1_0, t2, seg, fa, k, last; };
+    auto member_of = [&](long long item) -> int {
+        int lo = 0, hi = a0.ens_n - 1;   // last member whose first item is <= item
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (a0.ens_tile_start[mid] <= tile) lo = mid; else hi = mid - 1;
+            if (a0.ens_tile_start[mid] <= item) lo = mid; else hi = mid - 1;
         }
         return lo;
     };
-    // (a __grid_constant__ parameter may be addressed: it is not copied)
-    auto args_of = [&](long long tile, long long& lt) -> const SweepArgs* {
+    const int chunks = a0.seg_chunks;
+    long long nitems;
+    if constexpr (ENS) nitems = a0.ens_tile_start[a0.ens_n];
+    else nitems = CUT(a0.g, chunks).items();
+    const long long stride = (long long)gridDim.x * WPB;
+    // the item's first place; items of members that are not stepping are skipped whole
+    auto enter = [&](long long item) -> Place {
+        Place p;
+        p.a = &a0;
+        long long li = item;
         if constexpr (ENS) {
-            const int m = member_of(tile);
-            lt = tile - a0.ens_tile_start[m];
-            return a0.ens_tab + ((long long)m * a0.ens_stride + a0.ens_off + a0.ens_par[m]);
-        } else {
-            lt = tile;
-            return &a0;
-        }
-    };
-    // tile index -> (tile along the sweep, first line, plane); a single domain
-    // has fewer than 2^31 tiles, so 32-bit divisions serve
-    auto tile_coords = [](long long t, int ntx, int nty, int& tx, int& ty, int& tz) {
-        if constexpr (ENS) {
-            tx = (int)(t % ntx);
-            const long long r = t / ntx;
-            ty = (int)(r % nty);
-            tz = (int)(r / nty);
-        } else {
-            const unsigned u = (unsigned)t, r = u / (unsigned)ntx;
-            tx = (int)(u - r * (unsigned)ntx);
-            const unsigned z = r / (unsigned)nty;
-            ty = (int)(r - z * (unsigned)nty);
-            tz = (int)z;
-        }
-    };
-    long long ntiles;
-    if constexpr (ENS) {
-        ntiles = a0.ens_tile_start[a0.ens_n];
-    } else {
-        const Geo G = geo_of(a0.g);
-        const int nt2 = DIR == 2 ? a0.g.ny : a0.g.nz;
-        ntiles = (long long)G.ntx * G.nty * nt2;
-    }
-    // the first tile at or after t (stepping by the grid) of a member that is
-    // stepping; members that reached their end time are skipped whole
-    auto advance = [&](long long t) -> long long {
-        if constexpr (ENS) {
-            while (t < ntiles) {
-                const int m = member_of(t);
-                if (a0.ens_active[m]) return t;
+            while (item < nitems) {
+                const int m = member_of(item);
+                if (a0.ens_active[m]) {
+                    p.a = a0.ens_tab + ((long long)m * a0.ens_stride + a0.ens_off + a0.ens_par[m]);
+                    li = item - a0.ens_tile_start[m];
+                    break;
+                }
                 const long long end = a0.ens_tile_start[m + 1];
-                t += (end - t + gridDim.x - 1) / gridDim.x * gridDim.x;
+                item += (end - item + stride - 1) / stride * stride;
             }
         }
-        return t;
+        p.item = item;
+        p.t1_0 = p.t2 = p.seg = p.fa = p.last = 0;
+        p.k = -1;
+        if (item >= nitems) return p;
+        const CUT c(p.a->g, chunks);
+        // line groups fastest: neighbouring warps work on neighbouring lines
+        // (a sweep has fewer than 2^31 items, so 32-bit divisions serve)
+        const unsigned u = (unsigned)li, r = u / (unsigned)c.groups;
+        p.t1_0 = CUT::line0 + NL * (int)(u - r * (unsigned)c.groups);
+        const unsigned sg = r / (unsigned)c.nt2;
+        p.t2 = 3 + (int)(r - sg * (unsigned)c.nt2);
+        p.seg = (int)sg;
+        p.fa = CUT::f0 + (int)sg * (chunks * W - CUT::ov);
+        const int all = (c.n - p.fa) / W;   // chunk of the last interface n
+        p.last = all < chunks - 1 ? all : chunks - 1;
+        return p;
     };
-    const int tid = threadIdx.x;
-    // the compute threads' tile waits (a failure-detection test can make them
-    // give up at once); the drain in bail() below always keeps kWaitLimit
-    const uint32_t wait_limit = a0.wait_expire ? 0u : kWaitLimit;
-    // the thread that issues and tracks the tile copies: the block's last,
-    // whose warp has the least P1 work, so issuing does not delay P1
-    const bool issuer = tid == NT - 1;
+    auto after = [&](const Place& p) -> Place {
+        if (p.k < p.last) { Place q = p; ++q.k; return q; }
+        return enter(p.item + stride);
+    };
 
-    if (issuer) {
-        for (int k = 0; k < NBUF + NOB; ++k) mbar_init(&bars[k], 1);
+    if (lane == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
         fence_barrier_init();
     }
-    __syncthreads();
-
-    // TMA loads (the issuer only): the raw tile of `tile` into raw buffer b
-    // (which == 0) or its update operand into operand buffer b (which == 1).
-    auto issue = [&](long long gtile, int which, int b) -> bool {
-        long long tile;
-        const SweepArgs& a = *args_of(gtile, tile);
-        const Geo G = geo_of(a.g);
-        const int ntx = G.ntx, nty = G.nty;
-        int tx, ty, tz;
-        tile_coords(tile, ntx, nty, tx, ty, tz);
-        const int c0 = tx * T, t1_0 = line0 + ty * NL, t2 = 3 + tz;
-        int cc[4];
-        if (which == 0) {
-            if (DIR == 0) { cc[0] = c0; cc[1] = t1_0; cc[2] = t2; }
-            else if (DIR == 1) { cc[0] = t1_0; cc[1] = c0; cc[2] = t2; }
-            else { cc[0] = t1_0; cc[1] = t2; cc[2] = c0; }
-        } else {
-            if (DIR == 0) { cc[0] = c0 + 2; cc[1] = t1_0; cc[2] = t2; }
-            else if (DIR == 1) { cc[0] = t1_0; cc[1] = c0 + 3; cc[2] = t2; }
-            else { cc[0] = t1_0; cc[1] = t2; cc[2] = c0 + 3; }
-        }
-        cc[3] = 0;
-        if (cc[0] & 1) {   // never issue a misaligned tensor copy
-            atomicOr(a.status, HOW_STATUS_TMA_ALIGN);
+    __syncwarp();
+    bool issued = true;            // lane 0's view
+    unsigned par = 0u, pend = 0u;  // per barrier: phase parity, copy in flight (lane 0's view)
+    // TMA loads (lane 0): the new cells of place p (which == 0), or the update
+    // operand of its chunk (which == 1): cells fb+2 .. fb+W+1
+    auto issue = [&](const Place& p, int which) -> bool {
+        const int fb = p.fa + p.k * W;
+        const int along = which == 0 ? fb + 5 : DIR == 0 ? fb + 1 : fb + 2;
+        const int c0 = DIR == 0 ? along : p.t1_0;
+        const int c1 = DIR == 0 ? p.t1_0 : DIR == 1 ? along : p.t2;
+        const int c2 = DIR == 2 ? along : p.t2;
+        if (c0 & 1) {   // never issue a misaligned tensor copy
+            atomicOr(p.a->status, HOW_STATUS_TMA_ALIGN);
             return false;
         }
-        fence_proxy_async_smem();
-        if (which == 0) {
-            mbar_arrive_expect_tx(&bars[b], TL::in_bytes);
-            tma_load_4d(sm + TL::bQ + b * align_up(8 * TL::NQ, 128), &a.tm_in, &bars[b], cc[0], cc[1], cc[2], cc[3]);
-        } else {
-            mbar_arrive_expect_tx(&bars[NBUF + b], TL::out_bytes);
-            tma_load_4d(sm + TL::bO + b * align_up(8 * TL::NO, 128), &a.tm_out, &bars[NBUF + b], cc[0], cc[1], cc[2],
-                        cc[3]);
-        }
+        pend |= 1u << which;
+        mbar_arrive_expect_tx(&bars[which], which == 0 ? M::raw_bytes : M::op_bytes);
+        tma_load_4d(sm + (which == 0 ? M::bRaw : M::bOp), which == 0 ? &p.a->tm_in : &p.a->tm_out, &bars[which], c0,
+                    c1, c2, 0);
         return true;
     };
-    // MODE 1: the routing pass's decisions for tile t's faces and one more on
-    // each side of every line (faces -1 .. F), fetched by asynchronous 4-byte
-    // copies of the aligned words that hold them into decision set `slot`,
-    // one tile ahead so their latency hides behind a whole tile.  Every
-    // thread commits one group per call (empty past the last tile); returns
-    // the byte of this thread's word, -1 for no face.
-    auto fetch_dec = [&](long long t, int slot) -> int {
-        int shift = -1;
-        if constexpr (MODE == 1) {
-            static_assert(NL * FE <= NT, "one fetched decision per thread");
-            if (tid < NL * FE && t < ntiles) {
-                const Geo G = geo_of(a0.g);
-                int tx, ty, tz;
-                tile_coords(t, G.ntx, G.nty, tx, ty, tz);
-                const int l = tid / FE, f = tid % FE - 1;
-                const int t1 = line0 + ty * NL + l, iface = tx * T + f;
-                if (t1 >= 3 && t1 <= G.nt1 + 2 && iface >= 0 && iface <= G.n) {
-                    const unsigned char* src = a0.route_next + route_line(a0.g, DIR, t1, 3 + tz) + (iface + 2);
-                    shift = (int)(reinterpret_cast<uintptr_t>(src) & 3u);
-                    cp_async4(&sDecW[slot * DWS + tid],
-                              reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(3)));
-                }
-            }
-            cp_async_commit();
+    // the lanes' tile waits are bounded (a failure-detection test can make
+    // them give up at once); on expiry the warp leaves, lane 0 after a
+    // bounded wait for its copies in flight
+    const uint32_t wait_limit = a0.wait_expire ? 0u : kWaitLimit;
+    auto arrived = [&](int which) -> bool {
+        const bool ok = issued && mbar_wait_bounded(&bars[which], (par >> which) & 1u, wait_limit);
+        if (__all_sync(ALL, ok)) {
+            par ^= 1u << which;
+            pend &= ~(1u << which);
+            return true;
         }
-        return shift;
+        if (lane == 0) {
+            atomicOr(a0.status, HOW_STATUS_TMA_TIMEOUT);
+            for (int b = 0; b < 2; ++b)
+                if ((pend >> b) & 1u) mbar_wait_bounded(&bars[b], (par >> b) & 1u, kWaitLimit);
+        }
+        return false;
     };
 
+    // optional per-phase cycle accounting of lane 0 (prof != nullptr), summed
+    // in shared memory and added to the counters at the end
+    __shared__ unsigned long long s_prof[WPB][12];
+    const bool timed = a0.prof != nullptr && lane == 0;
+    if (timed)
+        for (int k = 0; k < 12; ++k) s_prof[warp][k] = 0ull;
+    unsigned tprev = (unsigned)clock();
+    auto mark = [&](int ph) {
+        if (timed) {
+            const unsigned now = (unsigned)clock();
+            s_prof[warp][ph] += now - tprev;
+            if (ph == 10) ++s_prof[warp][11];   // chunks
+            tprev = (unsigned)clock();
+        }
+    };
     // a single domain's dt / d is one value for the whole launch
     const double dtdl_launch = ENS ? 0.0 : *a0.dtdl;
-    long long tile = advance(blockIdx.x);
-    int buf = 0;               // raw buffer of this tile
-    int ob = 0;                // update operand buffer and decision set of this tile
-    uint32_t par_bits = 0u;    // phase parity per barrier (bit k)
-    uint32_t pend_bits = 0u;   // copies in flight per barrier (the issuer's view, bit k)
-    bool issued_ok = true;
-    if (issuer && tile < ntiles) {
-        // this tile's raw tile and update operand, and the raw tiles of the
-        // next NBUF - 1 tiles of this block
-        issued_ok = issue(tile, 0, 0) && issue(tile, 1, 0);
-        pend_bits = issued_ok ? (1u | (1u << NBUF)) : 0u;
-        long long ahead = advance(tile + gridDim.x);
-        for (int k = 1; k < NBUF - 1 && ahead < ntiles; ++k) {
-            issued_ok = issue(ahead, 0, k) && issued_ok;
-            pend_bits |= 1u << k;
-            ahead = advance(ahead + gridDim.x);
-        }
-    }
-    int dec_cur = fetch_dec(tile, 0);   // this tile's decision words (MODE 1)
-    // On a failed wait the whole block leaves together; the issuer first waits
-    // (bounded) for the copies it still has in flight.
-    auto bail = [&]() {
-        if (issuer) {
-            atomicOr(a0.status, HOW_STATUS_TMA_TIMEOUT);
-            for (int k = 0; k < NBUF + NOB; ++k)
-                if ((pend_bits >> k) & 1u) mbar_wait_bounded(&bars[k], (par_bits >> k) & 1u, kWaitLimit);
-        }
-    };
-    // optional per-phase cycle accounting of thread 0 (prof != nullptr)
-    long long tprev = clock64();
-    auto mark = [&](int ph) {
-        if (a0.prof != nullptr && tid == 0) {
-            const long long now = clock64();
-            atomicAdd(a0.prof + ph, (unsigned long long)(now - tprev));
-            if (ph == 10) atomicAdd(a0.prof + 11, 1ull);   // tiles
-            tprev = now;
-        }
-    };
-    for (; tile < ntiles; tile = advance(tile + gridDim.x)) {
-        long long ltile;
-        const SweepArgs& a = *args_of(tile, ltile);
-        const Grid& g = a.g;
-        const Geo G = geo_of(g);
-        const int n = G.n, nt1 = G.nt1, ntx = G.ntx, nty = G.nty;
-        const long long sstride = G.sstride;
-        const double gam = a.gam;
-        const R gamR = R(a.gam);
-        const R gam0 = R(1) - gamR, gam1 = R(0.5) * (gamR - R(1));
-        const R gam2 = (gamR - R(2)) / (gamR - R(1));
-        int tx, ty, tz;
-        tile_coords(ltile, ntx, nty, tx, ty, tz);
-        const int c0 = tx * T;                       // padded index of tile cell 0
-        const int t1_0 = line0 + ty * NL;
-        const int t2 = 3 + tz;
-        auto line_off = [&](int l) -> long long {
-            const int t1 = t1_0 + l;
-            if (DIR == 0) return g.idx(0, t1, t2);
-            if (DIR == 1) return g.idx(t1, 0, t2);
-            return g.idx(t1, t2, 0);
-        };
-        auto line_ok = [&](int l) -> bool { return t1_0 + l >= 3 && t1_0 + l <= nt1 + 2; };
-        // the line's first byte in the router's per-face arrays (route_line)
-        auto rline = [&](int l) -> long long { return route_line(g, DIR, t1_0 + l, t2); };
-        const double* sQ = reinterpret_cast<const double*>(sm + TL::bQ + buf * align_up(8 * TL::NQ, 128));
-        const double* sO = reinterpret_cast<const double*>(sm + TL::bO + ob * align_up(8 * TL::NO, 128));
-        // raw conserved of line variable v at (line l, tile cell c); box order
-        // x: [var][line][cell], y/z: [var][cell][line]
-        auto qraw = [&](int v, int l, int c) -> double {
-            const int gv = perm_of(DIR, v);
-            return DIR == 0 ? sQ[(gv * NL + l) * C + c] : sQ[(gv * C + c) * NL + l];
-        };
-        auto oraw = [&](int gv, int l, int ct) -> double {
-            return DIR == 0 ? sO[(gv * NL + l) * TO + ct + 1] : sO[(gv * TO + ct) * NL + l];
-        };
+    unsigned n_full = 0, n_cheap = 0;   // routed interfaces of this warp
 
-        // ------------------------------------------------------------ P0
-        {
-            const bool ok = issued_ok && mbar_wait_bounded(&bars[buf], (par_bits >> buf) & 1u, wait_limit);
-            if (__syncthreads_or(!ok)) { bail(); return; }   // results void; host sees the status
+    Place p = enter((long long)blockIdx.x * WPB + warp);
+    if (lane == 0 && p.item < nitems) issued = issue(p, 0);
+    while (p.item < nitems) {
+        const SweepArgs& a = *p.a;
+        const Grid& g = a.g;
+        const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
+        const int nt1 = DIR == 0 ? g.ny : g.nx;
+        const int fb = p.fa + p.k * W, f = fb + j;   // the chunk's first interface, the lane's
+        const int t1 = p.t1_0 + l;
+        const bool line_ok = t1 >= 3 && t1 <= nt1 + 2;
+        const long long sstride = DIR == 0 ? 1ll : DIR == 1 ? (long long)g.pitch : (long long)g.pitch * g.P1;
+        const long long line = DIR == 0 ? g.idx(0, t1, p.t2) : DIR == 1 ? g.idx(t1, 0, p.t2) : g.idx(t1, p.t2, 0);
+        const long long at = line + (long long)(f + 2) * sstride;   // the face, and the cell left of it
+        // faces this segment owns: all from its second (the x sweep: third)
+        // interface on, and face 0
+        const bool owned = line_ok && f <= n && f >= (p.seg == 0 ? 0 : p.fa + CUT::ov);
+        const double gam = a.gam, gm1 = gam - 1.0;
+
+        // -------------------------------------------------------------- load
+        if (!arrived(0)) return;   // results void; host sees the status
+        double q[8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            const int gv = perm_of(DIR, v);
+            q[v] = DIR == 0 ? sRaw[(gv * NL + l) * W + j] : sRaw[gv * 32 + lane];
         }
-        par_bits ^= 1u << buf;
-        pend_bits &= ~(1u << buf);
-        const long long next = advance(tile + gridDim.x);
+        __syncwarp();   // every read of the raw tile, and of the window's new columns, is done
         {
-            // the raw tile NBUF - 1 tiles ahead, into the buffer the previous
-            // tile used, and the next tile's update operand into the operand
-            // buffer the previous tile used (every read of both ended with
-            // that tile's last barrier)
-            long long ahead = next;
-            for (int k = 2; k < NBUF; ++k) ahead = advance(ahead + gridDim.x);
-            const int nb = (buf + NBUF - 1) % NBUF;
-            if (issuer && ahead < ntiles) {
-                issued_ok = issue(ahead, 0, nb) && issued_ok;
-                pend_bits |= 1u << nb;
-            }
-            if (issuer && next < ntiles) {
-                issued_ok = issue(next, 1, ob ^ 1) && issued_ok;
-                pend_bits |= 1u << (NBUF + (ob ^ 1));
+            const Place nx = after(p);
+            if (lane == 0) {
+                fence_proxy_async_smem();
+                if (p.k >= 0) issued = issue(p, 1) && issued;
+                if (nx.item < nitems) issued = issue(nx, 0) && issued;
             }
         }
-        const int dec_next = fetch_dec(next, ob ^ 1);   // the next tile's decisions (MODE 1)
-        // this stage's dt / d (per member in an ensemble), used in P5
-        const double dtdl_tile = ENS ? *a.dtdl : dtdl_launch;
+        // MODE 1: the routing pass's decisions of the lane's face and its two
+        // neighbours along the sweep (decisions formed once per step stay
+        // valid while a feature moves by up to one cell)
+        bool flagged = false;
+        if constexpr (MODE == 1) {
+            if (p.k >= 0 && line_ok) {
+                const unsigned char* d = a.route_next + route_line(g, DIR, t1, p.t2) + (f + 2);
+                unsigned any = 0u;
+#pragma unroll
+                for (int s = -1; s <= 1; ++s)
+                    if (f + s >= 0 && f + s <= n) any |= d[s];
+                flagged = any != 0u;
+            }
+        }
+        // this stage's dt / d (per member in an ensemble)
+        const double dtdl = ENS ? *a.dtdl : dtdl_launch;
         mark(0);
 
-        // P2a: eigen-system scalars of interface t from the arithmetic mean of
-        // its two cells' primitives (src/ssprk.cpp:610-660)
-        auto p2a_core = [&](int t, double mrho, double mvx, double mvy, double mvz, double mBx, double mBy,
-                            double mBz, double mHH) {
-            const R rho = R(mrho), vx = R(mvx), vy = R(mvy), vz = R(mvz);
-            const R Bx = R(mBx), By = R(mBy), Bz = R(mBz), HH = R(mHH);
-            const R vv2 = vx * vx + vy * vy + vz * vz;
-            const R BB2 = Bx * Bx + By * By + Bz * Bz;
-            const R isqr = Math<R>::rsq(rho);
-            const R irho = isqr * isqr;
-            const R bbn2 = BB2 * irho;
-            const R bnx2 = Bx * Bx * irho;
-            const R cs2 = (gamR - R(1)) * (HH - R(0.5) * (vv2 + bbn2));
-            const R cs = Math<R>::sq(fmax(R(0), cs2));
-            const R root = Math<R>::sq(fmax(R(0), (bbn2 + cs2) * (bbn2 + cs2) - R(4) * bnx2 * cs2));
-            const R lf = Math<R>::sq(fmax(R(0), R(0.5) * (bbn2 + cs2 + root)));
-            const R la = fabs(Bx) * isqr;
-            const R ls = Math<R>::sq(fmax(R(0), R(0.5) * (bbn2 + cs2 - root)));
-            const R Bt2 = By * By + Bz * Bz;
-            R bty, btz;
-            if (Bt2 >= R(1.0e-30)) { const R ib = Math<R>::rsq(Bt2); bty = By * ib; btz = Bz * ib; }
-            else { bty = R(0.70710678118654752440); btz = R(0.70710678118654752440); }
-            R af, as;
-            const R df = lf * lf - ls * ls;
-            if (df >= R(1.0e-30)) {
-                const R idf = Math<R>::rsq(df);
-                af = Math<R>::sq(fmax(R(0), cs2 - ls * ls)) * idf;
-                as = Math<R>::sq(fmax(R(0), lf * lf - cs2)) * idf;
-            } else { af = R(1); as = R(1); }
-            R* S = sS + t;
-            S[S_VX * NI] = vx; S[S_VY * NI] = vy; S[S_VZ * NI] = vz;
-            S[S_BY * NI] = By; S[S_BZ * NI] = Bz; S[S_VV2 * NI] = vv2;
-            S[S_CS * NI] = cs; S[S_CS2 * NI] = cs2; S[S_LF * NI] = lf; S[S_LS * NI] = ls;
-            S[S_AF * NI] = af; S[S_AS * NI] = as; S[S_BTY * NI] = bty; S[S_BTZ * NI] = btz;
-            S[S_SGNBX * NI] = sign1(Bx);
-            S[S_SQR * NI] = rho * isqr; S[S_ISQR * NI] = isqr;
-            S[S_SGNBT * NI] = (By != R(0)) ? sign1(By) : sign1(Bz);
-            S[S_FLIP * NI] = (cs >= la) ? R(1) : R(0);
-            S[S_BTV * NI] = bty * vy + btz * vz;
-            S[S_ICS2 * NI] = Math<R>::rcp(cs2);
-        };
-        // entry k of the interface list (every interface in the plain method),
-        // from the primitives P1 stored
-        auto p2a_item = [&](int k) {
-            const int t = ROUTED ? sList[k] : k;
-            const int c = (t / F) * C + t % F + 2;
-            p2a_core(t, 0.5 * (sP[0 * NLC + c] + sP[0 * NLC + c + 1]), 0.5 * (sP[1 * NLC + c] + sP[1 * NLC + c + 1]),
-                     0.5 * (sP[2 * NLC + c] + sP[2 * NLC + c + 1]), 0.5 * (sP[3 * NLC + c] + sP[3 * NLC + c + 1]),
-                     0.5 * (sP[4 * NLC + c] + sP[4 * NLC + c + 1]), 0.5 * (sP[5 * NLC + c] + sP[5 * NLC + c + 1]),
-                     0.5 * (sP[6 * NLC + c] + sP[6 * NLC + c + 1]), 0.5 * (sP[8 * NLC + c] + sP[8 * NLC + c + 1]));
-        };
-
-        // ------------------------------------------------------------ P1
-        // two threads per cell: the first forms primitives and fluxes, the
-        // second the eigenvalues (both from the same primitive arithmetic)
-        // primit (src/ssprk.cpp:479-512) of tile cell (l, cc): v from the
-        // unfloored density, floors on rho and p with E recomputed
-        struct Prim { double rho, irho, vx, vy, vz, Bx, By, Bz, EE, pg, vv2, BB2, Mx, My, Mz; };
-        auto primit = [&](int l, int cc) -> Prim {
-            Prim o;
-            const double DD = qraw(0, l, cc);
-            o.Mx = qraw(1, l, cc); o.My = qraw(2, l, cc); o.Mz = qraw(3, l, cc);
-            o.Bx = qraw(4, l, cc); o.By = qraw(5, l, cc); o.Bz = qraw(6, l, cc);
-            o.EE = qraw(7, l, cc);
-            o.rho = DD;
-            o.irho = 1.0 / o.rho;
-            o.vx = o.Mx * o.irho; o.vy = o.My * o.irho; o.vz = o.Mz * o.irho;
-            o.vv2 = o.vx * o.vx + o.vy * o.vy + o.vz * o.vz;
-            o.BB2 = o.Bx * o.Bx + o.By * o.By + o.Bz * o.Bz;
-            o.pg = (gam - 1.0) * (o.EE - 0.5 * (o.rho * o.vv2 + o.BB2));
-            if (o.rho < a.rhomin || o.pg < a.pgmin) {
-                o.rho = fmax(a.rhomin, o.rho);
-                o.pg = fmax(a.pgmin, o.pg);
-                o.EE = o.pg / (gam - 1.0) + 0.5 * (o.rho * o.vv2 + o.BB2);
-                o.irho = 1.0 / o.rho;
+        // -------------------------------------------------------------- cell
+        CellValues<R> cv;
+        cell_values<MODE>(q, gam, a.rhomin, a.pgmin, cv);
+        {
+            constexpr int nP = M::HP * NL, nB = M::HB * NL, nD = M::HD * NL, nL = M::HL * NL;
+            const double By = q[5], Bz = q[6];
+            sP[0 * CP + nP] = cv.rho; sP[1 * CP + nP] = cv.vx; sP[2 * CP + nP] = By; sP[3 * CP + nP] = Bz;
+            sP[4 * CP + nP] = cv.HH;
+            sB[0 * CB + nB] = cv.vy; sB[1 * CB + nB] = cv.vz; sB[2 * CB + nB] = q[4];
+#pragma unroll
+            for (int r = 0; r < 7; ++r) sF[r * CP + nP] = cv.F[r];
+#pragma unroll
+            for (int m = 0; m < 7; ++m) sL[m * CL + nL] = cv.lam[m];
+            if constexpr (MODE != 0) {
+#pragma unroll
+                for (int r = 0; r < M::NCF; ++r) sC[r * CL + nL] = cv.cf[r];
             }
-            return o;
-        };
-        for (int tt = tid; tt < 2 * NLC; tt += blockDim.x) {
-            const bool eig = tt >= NLC;
-            const int t = eig ? tt - NLC : tt;
-            const int l = t / C, cc = t % C;
-            const Prim u = primit(l, cc);
-            const double rho = u.rho, irho = u.irho, vx = u.vx, vy = u.vy, vz = u.vz;
-            const double Bx = u.Bx, By = u.By, Bz = u.Bz, EE = u.EE, pg = u.pg, vv2 = u.vv2, BB2 = u.BB2;
-            const double Mx = u.Mx, My = u.My, Mz = u.Mz;
-            if (!eig) {
-                const double HH = (EE + pg) * irho;
-                sP[0 * NLC + t] = rho; sP[1 * NLC + t] = vx; sP[2 * NLC + t] = vy; sP[3 * NLC + t] = vz;
-                sP[4 * NLC + t] = Bx; sP[5 * NLC + t] = By; sP[6 * NLC + t] = Bz; sP[7 * NLC + t] = pg;
-                sP[8 * NLC + t] = HH;
-                // eigenst centre fluxes (src/ssprk.cpp:561-593), with DD, EE the floored values
-                const double pt = pg + 0.5 * BB2;
-                const double vdB = vx * Bx + vy * By + vz * Bz;
-                double* U = sUst + t * 14;
-                double* Fc = sFc + t * 7;
-                Fc[0] = U[0] = rho * vx;                 // DD (floored) * vx
-                Fc[1] = U[1] = Mx * vx + pt - Bx * Bx;
-                Fc[2] = U[2] = My * vx - Bx * By;
-                Fc[3] = U[3] = Mz * vx - Bx * Bz;
-                Fc[4] = U[4] = By * vx - Bx * vy;
-                Fc[5] = U[5] = Bz * vx - Bx * vz;
-                Fc[6] = U[6] = (EE + pt) * vx - Bx * vdB;
-                U[7] = rho; U[8] = Mx; U[9] = My; U[10] = Mz; U[11] = By; U[12] = Bz; U[13] = EE;
-            } else {
-                // eigenvalues (src/ssprk.cpp:561-593), in the working type R:
-                // FP64 for the plain method, FP32 in the mixed one (where they
-                // feed only the FP32 characteristic part)
-                const R irR = R(irho);
-                const R bbn2 = R(BB2) * irR;
-                const R bnx2 = R(Bx * Bx) * irR;
-                const R cs2 = fmax(R(0), gamR * fabs(R(pg) * irR));
-                const R root = Math<R>::sq(fmax(R(0), (bbn2 + cs2) * (bbn2 + cs2) - R(4) * bnx2 * cs2));
-                const R lf = Math<R>::sq(fmax(R(0), R(0.5) * (bbn2 + cs2 + root)));
-                if constexpr (MODE != 0) {
-                    // the routing features' cell values, once per cell (the
-                    // guard of MODE 1 needs density and pressure only)
-                    sCF[0 * NLC + t] = (float)rho;
-                    sCF[1 * NLC + t] = (float)pg;
-                    if constexpr (MODE != 1) {
-                        sCF[2 * NLC + t] = sqrtf((float)BB2);
-                        sCF[3 * NLC + t] = sqrtf((float)vv2);
-                        sCF[4 * NLC + t] = (float)lf;
-                    }
-                }
-                const R la = Math<R>::sq(fmax(R(0), bnx2));
-                const R ls = Math<R>::sq(fmax(R(0), R(0.5) * (bbn2 + cs2 - root)));
-                const R vxR = R(vx);
-                // |lambda_m|: every reader takes the magnitude (the LLF speeds)
-                sA[0 * NLC + t] = fabs(vxR - lf); sA[1 * NLC + t] = fabs(vxR - la);
-                sA[2 * NLC + t] = fabs(vxR - ls); sA[3 * NLC + t] = fabs(vxR);
-                sA[4 * NLC + t] = fabs(vxR + ls); sA[5 * NLC + t] = fabs(vxR + la);
-                sA[6 * NLC + t] = fabs(vxR + lf);
+            // differences of (F, q_proj) to the cell before, formed in FP64
+            // and stored in the working type.  The cell before: from the
+            // window, but momentum and energy from the neighbouring lane (or
+            // what the last lanes of the chunk before left)
+            double u[4] = {q[1], q[2], q[3], cv.EE}, before[14];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const double up = __shfl_up_sync(ALL, u[v], NL);
+                before[v == 3 ? 13 : 8 + v] = j == 0 ? sU[v * NL] : up;
             }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 7; ++r) before[r] = sF[r * CP + nP - NL];
+            before[7] = sP[0 * CP + nP - NL]; before[11] = sP[2 * CP + nP - NL]; before[12] = sP[3 * CP + nP - NL];
+            const double now[14] = {cv.F[0], cv.F[1], cv.F[2], cv.F[3], cv.F[4], cv.F[5], cv.F[6],
+                                    cv.rho, q[1], q[2], q[3], By, Bz, cv.EE};
+#pragma unroll
+            for (int v = 0; v < 14; ++v) sD[v * CD + nD] = R(now[v] - before[v]);
+            if (j == W - 1) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) sU[v * NL] = u[v];
+            }
+            __syncwarp();
         }
-        __syncthreads();
         mark(1);
 
-        // ------------------------------------------------------------ P1b
-        // cell differences of (F, q_proj) along each line, formed in FP64 and
-        // stored in the working type; shared by all 7 fields
-        for (int t = tid; t < NLC * 14; t += blockDim.x) {
-            const int c = (t / 14) % C;
-            sD[t] = (c + 1 < C) ? R(sUst[t + 14] - sUst[t]) : R(0);
-        }
-        if constexpr (MODE != 0) {
-            if (tid < 2) s_cnt[tid] = 0u;
-            if (tid == 0) s_nfull = 0;
-        }
-        if constexpr (MODE == 1) {
-            // this tile's decision words (fetched one tile ago) have arrived:
-            // keep this thread's byte
-            cp_async_wait_prior();
-            if (tid < NL * FE) {
-                int* w = sDecW + ob * DWS + tid;
-                *w = dec_cur < 0 ? 0 : (int)((((unsigned int)*w) >> (8 * dec_cur)) & 0xffu);
+        if (p.k >= 0) {
+            // ---------------------------------------------------------- face
+            double fl[7];   // the interface's flux, rows rho, Mx, My, Mz, By, Bz, E of the line frame
+            bool full = true;
+            if constexpr (ROUTED) {
+                float rr[6], pp[6];
+#pragma unroll
+                for (int s = 0; s < 6; ++s) { rr[s] = sC[s * NL]; pp[s] = sC[CL + s * NL]; }
+                // the hard guard on this stage's state, whatever the stage
+                // the network's decisions were formed at
+                full = flagged || router_guard_rp(rr, pp, (float)a.rhomin, (float)a.pgmin, a.guard_jump, a.guard_floor);
+                const unsigned mf = __ballot_sync(ALL, owned && full), mc = __ballot_sync(ALL, owned && !full);
+                n_full += __popc(mf);
+                n_cheap += __popc(mc);
+                if constexpr (MODE == 2) {
+                    if (owned) a.route_next[route_line(g, DIR, t1, p.t2) + (f + 2)] = (unsigned char)(full ? 1 : 0);
+                }
             }
-        }
-        __syncthreads();
-        mark(2);
+            // the stage input of the cell left of the interface, which the
+            // first sweep of a stage combines with the RK base (issued before
+            // the back-projection, used at the update)
+            double prev[8];
+            auto load_prev = [&] {
+                if (a.mode == 1 && owned && f >= 1) {
+                    const double* in = a.qprev + at;
+#pragma unroll
+                    for (int gv = 0; gv < 8; ++gv, in += g.fs) prev[line_var(DIR, gv)] = *in;
+                }
+            };
+            float lab_w = 0.0f, lab_f = 0.0f;   // MODE 3: largest weight and flux departures
 
-        // ------------------------------------------------------------ PR
-        // routing: features of every interface, the hard guard, the network
-        // (MODE 1), and the compacted list of interfaces that get full WENO
-        int nfull = NLF;
-        if constexpr (MODE != 0) {
-            // features of interface t (tile-local), its guard and its flatness
-            auto row_features = [&](int t, float* ft, bool& flat, float& prior) -> bool {
-                const int l = t / F, f = t % F;
-                StencilCell sc[6];
+            // a warp takes the full path when one of its faces does (shocks
+            // are surfaces: its 32 faces are neighbours), the linear one when
+            // one of its faces does; a face keeps the result of its own
+            if (!ROUTED || __any_sync(ALL, full)) {
+                FaceValues<R> fv;
+                face_values<NL, CP, CB, CD, CL, MODE>(sP, sB, sD, sL, R(gam), R(a.gam2), fv, load_prev);
+                if constexpr (MODE == 3) lab_w = fv.departure;
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int cc = l * C + f + k;
-                    sc[k] = StencilCell{sCF[0 * NLC + cc], sCF[1 * NLC + cc], sCF[2 * NLC + cc], sCF[3 * NLC + cc],
-                                        sCF[4 * NLC + cc]};
-                }
-                // the prior-stage feature is held at 0: fed back from the
-                // network's own decisions it locked smooth flows at full WENO
-                prior = 0.0f;
-                return router_features(sc, prior, (float)a.rhomin, (float)a.pgmin, a.guard_jump, a.guard_floor, ft,
-                                       &flat);
-            };
-            // Lax-Friedrichs speed of the linear flux: the stencil's largest |lambda|
-            auto row_amx = [&](int t) {
-                const int cb = (t / F) * C + t % F;
-                R amx = fmax(sA[0 * NLC + cb], sA[6 * NLC + cb]);
-#pragma unroll
-                for (int k = 1; k < 6; ++k) amx = fmax(amx, fmax(sA[0 * NLC + cb + k], sA[6 * NLC + cb + k]));
-                sAmx[t] = amx;
-            };
-            if constexpr (MODE == 1) {
-                // decisions of the learned router, formed for the whole sweep by
-                // the routing pass (route_prepass.cu) before this launch
-                // a face takes full WENO when the pass flagged it or a neighbour
-                // along the sweep (decisions formed once per step stay valid
-                // while a feature moves by up to one cell)
-                bool owned = false, full = false;
-                if (tid < NLF) {
-                    const int l = tid / F, f = tid % F;
-                    const int* d = sDecW + ob * DWS + l * FE + f;   // faces f-1, f, f+1
-                    // the hard guard on this stage's state, whatever the stage
-                    // the network's decisions were formed at
-                    const bool guard = router_guard_rp(sCF + l * C + f, sCF + NLC + l * C + f, (float)a.rhomin,
-                                                       (float)a.pgmin, a.guard_jump, a.guard_floor);
-                    full = guard || (d[0] | d[1] | d[2]);
-                    sDec[tid] = full ? 1 : 0;
-                    // list of full-WENO interfaces: P2a-P4 treat each entry on
-                    // its own, so the order the atomic gives does not matter
-                    if (full) sList[atomicAdd(&s_nfull, 1)] = tid;
-                    row_amx(tid);
-                    // counted once per face: a tile's last face is the next
-                    // tile's first, owned by the lower tile unless it ends the line
-                    const int iface = c0 + f;
-                    owned = line_ok(l) && iface <= n && (f < T || iface == n);
-                }
-                const unsigned int mf = __ballot_sync(0xffffffffu, owned && full);
-                const unsigned int mc = __ballot_sync(0xffffffffu, owned && !full);
-                if ((tid & 31) == 0) {
-                    if (mf) atomicAdd(&s_cnt[0], (unsigned int)__popc(mf));
-                    if (mc) atomicAdd(&s_cnt[1], (unsigned int)__popc(mc));
-                }
-                __syncthreads();
-                mark(3);
-                mark(4);
-            } else {
-                for (int t = tid; t < NLF; t += blockDim.x) {
-                    float ft[kRouterNF];
-                    bool flat;
-                    float prior;
-                    const bool guard = row_features(t, ft, flat, prior);
-                    row_amx(t);
+                for (int r = 0; r < 7; ++r) {
+                    fl[r] = (double)fv.out[r] + sF[r * CP];
                     if constexpr (MODE == 3) {
+                        // label collection: what routing this face to the cheap
+                        // flux would change -- dt/dx |F_full - F_linear| for this
+                        // component, relative to the local size of its conserved
+                        // variable (density; rho (|v| + c) for momentum; sqrt(rho) c
+                        // for the field; the total energy), with
+                        // c^2 = (gam p + B^2) / rho at the mean state
+                        R amx = larger(sL[0], sL[6 * CL]), dF[5], dq[5];
 #pragma unroll
-                        for (int k = 0; k < kRouterNF; ++k) sFt[t * 6 + k] = ft[k];
-                        sDev[t] = 0.0f;
-                        sFlx[t] = 0.0f;
-                    }
-                    sDec[t] = MODE == 3 ? 1 : (guard ? 1 : 0);
-                    if constexpr (MODE == 2) {
-                        if (guard) sList[atomicAdd(&s_nfull, 1)] = t;
+                        for (int k = 1; k < 6; ++k) amx = larger(amx, larger(sL[k * NL], sL[6 * CL + k * NL]));
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) { dF[k] = sD[r * CD + k * NL]; dq[k] = sD[(7 + r) * CD + k * NL]; }
+                        const double lin = (double)linear_flux(dF, dq, amx);
+                        const double rho = fv.rho, v2 = 2.0 * fv.hvv, b2 = fv.bbn2 * fv.rho;
+                        const double pg = 0.5 * ((double)sC[CL + 2 * NL] + (double)sC[CL + 3 * NL]);
+                        const double c = sqrt((gam * pg + b2) / rho);
+                        const double scale = r == 0 ? rho
+                                           : r < 4 ? rho * (sqrt(v2) + c)
+                                           : r < 6 ? sqrt(rho) * c
+                                           : pg / gm1 + 0.5 * rho * v2 + 0.5 * b2;
+                        lab_f = fmaxf(lab_f, (float)(dtdl * fabs((double)fv.out[r] - lin) / scale));
                     }
                 }
-                __syncthreads();
-                mark(3);
             }
-            if constexpr (ROUTED) nfull = s_nfull;
-        }
-
-        mark(5);
-
-        // A routed tile with no full-WENO interface skips P2a-P3 and their
-        // barriers (nfull is the same for the whole block)
-        if (!ROUTED || nfull > 0) {
-        // ------------------------------------------------------------ P2a
-        for (int k = tid; k < nfull; k += blockDim.x) p2a_item(k);
-        __syncthreads();
-        mark(6);
-
-        // (the left rows and right columns are built where they are used: P3, P4)
-        mark(7);
-
-        // ------------------------------------------------------------ P3
-        // one interface ii, field m: left row, projection of its 5 cell
-        // differences, WENO flux
-        auto p3_one = [&](int m, int ii) {
-            const int l = ii / F, f = ii % F;
-            R L0[7];
-            eig_left_row<R, NI>(m, sS + ii, gam0, gam1, L0);
-            R dF0[5], dq0[5];
-            R amx0 = sA[m * NLC + l * C + f];
+            if constexpr (ROUTED) {
+                if (__all_sync(ALL, !full)) load_prev();   // (the full path was skipped)
+                if (__any_sync(ALL, !full)) {
+                    // Lax-Friedrichs speed of the linear flux: the stencil's largest |lambda|
+                    R amx = larger(sL[0], sL[6 * CL]);
 #pragma unroll
-            for (int cc = 0; cc < 5; ++cc) {
-                const int c = f + cc;
-                const V2* u = reinterpret_cast<const V2*>(sD + (l * C + c) * 14);
-                R pf = R(0), pq = R(0);
+                    for (int k = 1; k < 6; ++k) amx = larger(amx, larger(sL[k * NL], sL[6 * CL + k * NL]));
 #pragma unroll
-                for (int h = 0; h < 7; ++h) {
-                    // the seven (F, q) pairs of the difference, one 16-byte load each
-                    const V2 x = u[h];
-                    const int v0 = 2 * h, v1 = 2 * h + 1;   // components of D[14] = (dF[7], dq[7])
-                    if (v0 < 7) pf = (v0 == 0) ? L0[0] * x.x : pf + L0[v0] * x.x;
-                    else pq = (v0 == 7) ? L0[0] * x.x : pq + L0[v0 - 7] * x.x;
-                    if (v1 < 7) pf = pf + L0[v1] * x.y;
-                    else pq = (v1 == 7) ? L0[0] * x.y : pq + L0[v1 - 7] * x.y;
+                    for (int r = 0; r < 7; ++r) {
+                        R dF[5], dq[5];
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) { dF[k] = sD[r * CD + k * NL]; dq[k] = sD[(7 + r) * CD + k * NL]; }
+                        const double lin = (double)linear_flux(dF, dq, amx) + sF[r * CP];
+                        fl[r] = full ? fl[r] : lin;
+                    }
                 }
-                dF0[cc] = pf; dq0[cc] = pq;
-                amx0 = fmax(amx0, sA[m * NLC + l * C + c + 1]);
             }
             if constexpr (MODE == 3) {
-                R d0;
-                sFs[m * NI + ii] = weno_flux_d<R, true>(dF0, dq0, amx0, &d0);
-                atomicMax(reinterpret_cast<int*>(&sDev[ii]), __float_as_int((float)d0));
-            } else {
-                sFs[m * NI + ii] = weno_flux_d<R>(dF0, dq0, amx0);
-            }
-        };
-        // FP64 at five or more blocks per SM: one interface per thread, which
-        // holds one left row and one stencil in registers instead of two
-        constexpr bool P3_SINGLE = std::is_same<R, double>::value && MINB >= 5;
-        if constexpr (!ROUTED && P3_SINGLE) {
-            for (int t = tid; t < 7 * NLF; t += blockDim.x) p3_one(t % 7, t / 7);
-        } else if constexpr (!ROUTED) {
-            for (int t = tid; t < 7 * NL * NP; t += blockDim.x) {
-                const int m = t % 7, pr = t / 7;
-                const int l = pr / NP, p = pr % NP;
-                const int f0 = 2 * p;
-                const bool has1 = f0 + 1 < F;
-                const int i0 = l * F + f0;
-                const int i1 = has1 ? i0 + 1 : i0;
-                R L0[7], L1[7];
-                eig_left_row<R, NI>(m, sS + i0, gam0, gam1, L0);
-                eig_left_row<R, NI>(m, sS + i1, gam0, gam1, L1);
-                // interface f0 uses differences at cells f0..f0+4, f0+1 uses f0+1..f0+5
-                R dF0[5], dq0[5], dF1[5], dq1[5];
-                R amx0 = sA[m * NLC + l * C + f0];
-                R amx1 = sA[m * NLC + l * C + (f0 + 1 < C ? f0 + 1 : C - 1)];
+                // the records of owned faces of the sampled tiles (a hash of
+                // the index of the tile of 32 faces, 1 line in x and 2 lines
+                // x 16 faces in y and z, so the sample does not alias with the
+                // grid nor depend on how the sweep is cut)
+                if (owned) {
+                    a.route_next[route_line(g, DIR, t1, p.t2) + (f + 2)] = 0;
+                    constexpr int TL = DIR == 0 ? 1 : 2, TT = 32 / TL;
+                    const int ntx = (n + TT - 1) / TT;
+                    const int nty = DIR == 0 ? nt1 : (nt1 + 1 + TL - 1) / TL;
+                    const int tx = f / TT < ntx ? f / TT : ntx - 1, ty = DIR == 0 ? t1 - 3 : (t1 - 2) / TL;
+                    const long long tile = ((long long)(p.t2 - 3) * nty + ty) * ntx + tx;
+                    const unsigned long long hs = (unsigned long long)tile * 0x9E3779B97F4A7C15ull;
+                    if ((unsigned int)(hs >> 32) % a.collect_every == 0u) {
+                        StencilCell sc[6];
 #pragma unroll
-                for (int cc = 0; cc < 6; ++cc) {
-                    int c = f0 + cc;
-                    c = c < C - 1 ? c : C - 2;
-                    const V2* u = reinterpret_cast<const V2*>(sD + (l * C + c) * 14);
-                    R D[14];
+                        for (int s = 0; s < 6; ++s)
+                            sc[s] = StencilCell{sC[s * NL], sC[CL + s * NL], sC[2 * CL + s * NL], sC[3 * CL + s * NL],
+                                                sC[4 * CL + s * NL]};
+                        // the prior-stage feature is held at 0: fed back from the
+                        // network's own decisions it locked smooth flows at full WENO
+                        float ft[kRouterNF];
+                        bool flat;
+                        router_features(sc, 0.0f, (float)a.rhomin, (float)a.pgmin, a.guard_jump, a.guard_floor, ft, &flat);
+                        const unsigned int slot = atomicAdd(a.collect_n, 1u);
+                        if (slot < a.collect_cap) {
+                            float* rec = a.collect + 8ull * slot;
 #pragma unroll
-                    for (int h = 0; h < 7; ++h) { const V2 x = u[h]; D[2 * h] = x.x; D[2 * h + 1] = x.y; }
-                    const R av = sA[m * NLC + l * C + (c + 1)];
-                    if (cc <= 4) {
-                        R pf = L0[0] * D[0], pq = L0[0] * D[7];
-#pragma unroll
-                        for (int v = 1; v < 7; ++v) { pf += L0[v] * D[v]; pq += L0[v] * D[7 + v]; }
-                        dF0[cc] = pf; dq0[cc] = pq;
-                        amx0 = fmax(amx0, av);
-                    }
-                    if (cc >= 1) {
-                        R pf = L1[0] * D[0], pq = L1[0] * D[7];
-#pragma unroll
-                        for (int v = 1; v < 7; ++v) { pf += L1[v] * D[v]; pq += L1[v] * D[7 + v]; }
-                        dF1[cc - 1] = pf; dq1[cc - 1] = pq;
-                        amx1 = fmax(amx1, av);
+                            for (int k = 0; k < 6; ++k) rec[k] = ft[k];
+                            rec[6] = lab_w;
+                            rec[7] = lab_f;
+                        }
                     }
                 }
-                if constexpr (MODE == 3) {
-                    R d0, d1;
-                    sFs[m * NI + i0] = weno_flux_d<R, true>(dF0, dq0, amx0, &d0);
-                    atomicMax(reinterpret_cast<int*>(&sDev[i0]), __float_as_int((float)d0));
-                    if (has1) {
-                        sFs[m * NI + i1] = weno_flux_d<R, true>(dF1, dq1, amx1, &d1);
-                        atomicMax(reinterpret_cast<int*>(&sDev[i1]), __float_as_int((float)d1));
-                    }
-                } else {
-                    sFs[m * NI + i0] = weno_flux_d<R>(dF0, dq0, amx0);
-                    if (has1) sFs[m * NI + i1] = weno_flux_d<R>(dF1, dq1, amx1);
-                }
             }
-        } else {
-            // routed: pairs of entries of the compacted list, each with its own stencil
-            const int npair = (nfull + 1) / 2;
-            for (int t = tid; t < 7 * npair; t += blockDim.x) {
-                const int m = t % 7, p = t / 7;
-                const bool has1 = 2 * p + 1 < nfull;
-                const int i0 = sList[2 * p];
-                const int i1 = has1 ? sList[2 * p + 1] : i0;
-                p3_one(m, i0);
-                if (has1) p3_one(m, i1);
-            }
-        }
-        __syncthreads();
-        }   // P2a-P3
-        mark(8);
+            mark(8);
 
-        // ------------------------------------------------------------ P4
-        // per (interface, flux component): full WENO -> F_i + sum_m R(r,m) F^_m
-        // (back-projection in m order, src/ssprk.cpp:941-943); routed-linear
-        // interfaces -> the component-wise linear flux.  Components 4 and 5
-        // also form the CT terms (src/ssprk.cpp:973-993).
-        for (int t = tid; t < 7 * NLF; t += blockDim.x) {
-            const int r = t / NLF, i = t % NLF;
-            const int l = i / F, f = i % F;
-            const int c = l * C + f + 2;          // left cell of the interface
-            const double F2 = sFc[c * 7 + r];     // physical flux of that cell (central part)
-            double dF;
-            bool full = true;
-            if constexpr (ROUTED) full = sDec[i] != 0;
-            if (full) {
-                R Rr[7];
-                eig_right_row<R, NI>(r, sS + i, gam2, Rr);
-                R acc = R(0);
+            // CT terms (src/ssprk.cpp:973-993): flux plus the mean of B_n v_t
+            // over the two cells
+            if (owned) {
 #pragma unroll
-                for (int m = 0; m < 7; ++m) acc += Rr[m] * sFs[m * NI + i];
-                dF = (double)acc + F2;
-                if constexpr (MODE == 3) {
-                    // label collection: what routing this face to the cheap
-                    // flux would change -- dt/dx |F_full - F_linear| for this
-                    // component, relative to the local size of its conserved
-                    // variable (density; rho (|v| + c) for momentum; sqrt(rho) c
-                    // for the field; the total energy), with
-                    // c^2 = (gam p + B^2) / rho at the mean state
-                    R dFk[5], dqk[5];
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) {
-                        const int cc = l * C + f + k;
-                        dFk[k] = sD[cc * 14 + r];
-                        dqk[k] = sD[cc * 14 + 7 + r];
+                for (int c = 0; c < 2; ++c) {
+                    const double* v = sB + c * CB + NL;       // v_t1 or v_t2 of cell f+2
+                    const double* b = sB + 2 * CB + NL;       // B_n
+                    const double x1 = b[0] * v[0], x2 = b[NL] * v[NL];
+                    double avg;
+                    if (a.ct4) {
+                        // fourth-order midpoint value (-1, 9, 9, -1) / 16 over cells f+1 .. f+4
+                        avg = fm(9.0, x1 + x2, -(b[-NL] * v[-NL] + b[2 * NL] * v[2 * NL])) * 0.0625;
+                    } else {
+                        // the reference's two-point form (-0, 9, 9, -0) / 18
+                        avg = quot(fm(9.0, x1, 9.0 * x2), 18.0, 1.0 / 18.0);
                     }
-                    const double lin = (double)linear_flux_d<R>(dFk, dqk, sAmx[i]);
-                    const double rho = 0.5 * (sP[c] + sP[c + 1]);
-                    const double vx = 0.5 * (sP[NLC + c] + sP[NLC + c + 1]);
-                    const double vy = 0.5 * (sP[2 * NLC + c] + sP[2 * NLC + c + 1]);
-                    const double vz = 0.5 * (sP[3 * NLC + c] + sP[3 * NLC + c + 1]);
-                    const double bx = 0.5 * (sP[4 * NLC + c] + sP[4 * NLC + c + 1]);
-                    const double by = 0.5 * (sP[5 * NLC + c] + sP[5 * NLC + c + 1]);
-                    const double bz = 0.5 * (sP[6 * NLC + c] + sP[6 * NLC + c + 1]);
-                    const double pg = 0.5 * (sP[7 * NLC + c] + sP[7 * NLC + c + 1]);
-                    const double v2 = vx * vx + vy * vy + vz * vz, b2 = bx * bx + by * by + bz * bz;
-                    const double cs = sqrt((gam * pg + b2) / rho);
-                    const double scale = r == 0 ? rho
-                                       : r < 4 ? rho * (sqrt(v2) + cs)
-                                       : r < 6 ? sqrt(rho) * cs
-                                       : pg / (gam - 1.0) + 0.5 * rho * v2 + 0.5 * b2;
-                    const float dv = (float)(dtdl_tile * fabs((double)acc - lin) / scale);
-                    if (dv > 0.0f) atomicMax(reinterpret_cast<int*>(&sFlx[i]), __float_as_int(dv));
-                }
-            } else {
-                R dFk[5], dqk[5];
-#pragma unroll
-                for (int k = 0; k < 5; ++k) {
-                    const int cc = l * C + f + k;
-                    dFk[k] = sD[cc * 14 + r];
-                    dqk[k] = sD[cc * 14 + 7 + r];
-                }
-                dF = (double)linear_flux_d<R>(dFk, dqk, sAmx[i]) + F2;
-            }
-            sdF[r * NI + i] = dF;
-            const int iface = c0 + f;   // global interface index, face at padded iface + 2
-            const bool valid = line_ok(l) && iface <= n;
-            if (valid && (r == 4 || r == 5)) {
-                // CT terms: mean of B_n v_t over the two cells
-                const int vt = r == 4 ? 2 : 3;
-                const double x1 = sP[4 * NLC + c] * sP[vt * NLC + c];
-                const double x2 = sP[4 * NLC + c + 1] * sP[vt * NLC + c + 1];
-                const long long o = line_off(l) + (long long)(iface + 2) * sstride;
-                double avg;
-                if (a.ct4) {
-                    // fourth-order midpoint value (-1, 9, 9, -1) / 16 over cells c-1 .. c+2
-                    const double x0 = sP[4 * NLC + c - 1] * sP[vt * NLC + c - 1];
-                    const double x3 = sP[4 * NLC + c + 2] * sP[vt * NLC + c + 2];
-                    avg = (-x0 + 9.0 * x1 + 9.0 * x2 - x3) / 16.0;
-                } else {
-                    // the reference's two-point form (-0, 9, 9, -0) / 18
-                    avg = div_const(9.0 * x1 + 9.0 * x2, 18.0, 1.0 / 18.0);
-                }
-                (r == 4 ? a.cta : a.ctb)[o] = dF + avg;
-            }
-            if constexpr (MODE != 0) {
-                // a tile's last interface is also the next tile's first: the
-                // lower tile owns it unless it is the line's last face
-                if (valid && r == 0 && (f < T || iface == n)) {
-                    const long long o = rline(l) + (iface + 2);
-                    if constexpr (MODE == 2) {
-                        a.route_next[o] = (unsigned char)(full ? 1 : 0);
-                        atomicAdd(&s_cnt[full ? 0 : 1], 1u);
-                    }
+                    (c == 0 ? a.cta : a.ctb)[at] = fl[4 + c] + avg;
                 }
             }
-        }
-        __syncthreads();
-        if constexpr (MODE == 3) {
-            // the records of the tile's owned faces, once every component's
-            // flux departure is in (sampled tiles: a hash of the tile index,
-            // so the sample does not alias with the tile grid)
-            const unsigned long long hs = (unsigned long long)tile * 0x9E3779B97F4A7C15ull;
-            const bool sampled = (unsigned int)(hs >> 32) % a.collect_every == 0u;
-            for (int i = tid; i < NLF; i += blockDim.x) {
-                const int l = i / F, f = i % F, iface = c0 + f;
-                if (!(line_ok(l) && iface <= n && (f < T || iface == n))) continue;
-                a.route_next[rline(l) + (iface + 2)] = 0;
-                if (!sampled) continue;
-                const unsigned int slot = atomicAdd(a.collect_n, 1u);
-                if (slot < a.collect_cap) {
-                    float* rec = a.collect + 8ull * slot;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) rec[k] = sFt[i * 6 + k];
-                    rec[6] = sDev[i];
-                    rec[7] = sFlx[i];
-                }
-            }
-        }
-        if constexpr (ROUTED) {
-            if (tid == 0) {
-                atomicAdd(&a.route_count[0], (unsigned long long)s_cnt[0]);
-                atomicAdd(&a.route_count[1], (unsigned long long)s_cnt[1]);
+            mark(9);
 
+            // -------------------------------------------------------- update
+            double dfl[7];
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {
+                const double up = __shfl_up_sync(ALL, fl[r], NL);
+                dfl[r] = fl[r] - (j == 0 ? sX[r * NL] : up);
+            }
+            if (!arrived(1)) return;
+            // cell f+2, between this interface and the one before
+            if (owned && f >= 1) {
+                double* out = a.qout + at;
+#pragma unroll
+                for (int gv = 0; gv < 8; ++gv, out += g.fs) {
+                    const int v = line_var(DIR, gv);
+                    const double cur = DIR == 0 ? sOp[(gv * NL + l) * M::TO + j + 1] : sOp[gv * 32 + lane];
+                    double o = a.mode == 1 ? fm(a.k3, prev[v], a.k1 * cur) : cur;
+                    // (the flux rows skip line variable 4, the normal B)
+                    if (v != 4) o = fm(-dtdl, dfl[v < 4 ? v : v - 1], o);
+                    if (v != 4 || a.mode != 0) *out = o;
+                }
+            }
+            __syncwarp();   // every read of the operand tile and of sX is done
+            if (j == W - 1) {
+#pragma unroll
+                for (int r = 0; r < 7; ++r) sX[r * NL] = fl[r];
             }
         }
-        mark(9);
-
-        // ------------------------------------------------------------ P5
+        // the window's last cells become the history of the next chunk
+        __syncwarp();
         {
-            const bool ok = mbar_wait_bounded(&bars[NBUF + ob], (par_bits >> (NBUF + ob)) & 1u, wait_limit);
-            if (__syncthreads_or(!ok)) { bail(); return; }
-        }
-        par_bits ^= 1u << (NBUF + ob);
-        pend_bits &= ~(1u << (NBUF + ob));
-        const double dtdl = dtdl_tile;
-        for (int t = tid; t < 8 * NL * T; t += blockDim.x) {
-            int v, l, ct;
-            if (DIR == 0) { v = t / (NL * T); const int r = t % (NL * T); l = r / T; ct = r % T; }
-            else { v = t / (NL * T); const int r = t % (NL * T); ct = r / NL; l = r % NL; }
-            const int s = c0 + ct + 3;
-            if (!line_ok(l) || s > n + 2) continue;
-            const int rr = v < 4 ? v : v - 1;     // flux row of line variable v (v = 4: normal B)
-            const int fi = l * F + ct;
-            const double delta = (v == 4) ? 0.0 : -dtdl * (sdF[rr * NI + fi + 1] - sdF[rr * NI + fi]);
-            const int gv = perm_of(DIR, v);
-            const long long o = (long long)gv * g.fs + line_off(l) + (long long)s * sstride;
-            const double cur = oraw(gv, l, ct);   // q(iw) (accumulate) or the RK base
-            if (a.mode == 0) {
-                if (v != 4) a.qout[o] = cur + delta;
-            } else if (a.mode == 1) {
-                a.qout[o] = a.k1 * cur + a.k3 * qraw(v, l, ct + 3) + delta;
-            } else {
-                a.qout[o] = cur + delta;
+            MoveBack<double, 12, CP, M::HP * NL> pf;   // P and F rows are adjacent
+            MoveBack<double, 3, CB, M::HB * NL> vb;
+            MoveBack<R, 14, CD, M::HD * NL> d;
+            MoveBack<R, 7, CL, M::HL * NL> e;
+            pf.load(sP - lane, lane); vb.load(sB - lane, lane); d.load(sD - lane, lane); e.load(sL - lane, lane);
+            if constexpr (MODE != 0) {
+                MoveBack<float, M::NCF, CL, M::HL * NL> c;
+                c.load(sC - lane, lane);
+                c.store(sC - lane, lane);
             }
+            pf.store(sP - lane, lane); vb.store(sB - lane, lane); d.store(sD - lane, lane); e.store(sL - lane, lane);
         }
-        __syncthreads();   // every read of the update operand / raw tile is done
         mark(10);
-        buf = buf + 1 == NBUF ? 0 : buf + 1;
-        ob ^= 1;
-        dec_cur = dec_next;
-    }   // tile loop
+        p = after(p);
+    }
+    if (timed)
+        for (int k = 0; k < 12; ++k) atomicAdd(a0.prof + k, s_prof[warp][k]);
+    if constexpr (ROUTED) {
+        if (lane == 0) {
+            if (n_full) atomicAdd(&a0.route_count[0], (unsigned long long)n_full);
+            if (n_cheap) atomicAdd(&a0.route_count[1], (unsigned long long)n_cheap);
+        }
+    }
 }
 
 }  // namespace

@@ -1,5 +1,5 @@
 // sweep_kernels.cu -- single-domain launches of the fused directional sweep
-// (sweep_core.cuh): tile shapes, TMA tensor maps and the instantiations for
+// (sweep_core.cuh): work items, TMA tensor maps and the instantiations for
 // {FP64, mixed} x {plain, learned routing, guard-only routing, label
 // collection}.
 #include "sweep_core.cuh"
@@ -8,63 +8,72 @@ namespace how {
 
 namespace {
 
-template <int DIR, int NL, int T, int NT, typename R, int MINB, int MODE>
-void launch_one(Ctx& c, const SweepArgs& a) {
-    using TL = Tile<DIR, NL, T, R>;
-    constexpr size_t bytes = (MODE == 0 ? TL::bytes_plain : MODE == 1 ? TL::bytes_learned : TL::bytes_route) + 128;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(k_sweep<DIR, NL, T, NT, R, MINB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bytes);
-        attr_done = true;
-    }
-    const Grid& g = c.g;
+constexpr int kLines = 4;   // lines per warp: 32-byte rows in y and z
+
+// Length of the work items, in chunks: the one with the least time on the
+// busiest warp, rounds x (chunks + 1/4).  The quarter chunk stands for a
+// segment's first five cells, which have no interface yet.
+template <int DIR>
+int pick_chunks(const Grid& g, long long warps) {
+    using CUT = Cut<DIR, kLines>;
     const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
-    const int nt1 = DIR == 0 ? g.ny : g.nx;
-    const int nt2 = DIR == 2 ? g.ny : g.nz;
-    const long long ntx = (n + T - 1) / T;
-    const long long nty = DIR == 0 ? (nt1 + NL - 1) / NL : (nt1 + 1 + NL - 1) / NL;
-    const long long ntiles = ntx * nty * nt2;
-    int nsm = 148, occ = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
+    const int most = (n - CUT::f0) / CUT::W + 1;
+    int best = 1;
+    double best_t = 0.0;
+    for (int s = 1; s <= most; ++s) {
+        const long long rounds = (CUT(g, s).items() + warps - 1) / warps;
+        const double t = (double)rounds * (s + 0.25);
+        if (s == 1 || t < best_t) { best = s; best_t = t; }
+    }
+    return best;
+}
+
+template <int DIR, int WPB, typename R, int MINB, int MODE>
+void launch_one(Ctx& c, SweepArgs& a) {
+    constexpr int bytes = WPB * WarpMem<DIR, kLines, R, MODE>::bytes + 128;
+    const auto kern = k_sweep<DIR, kLines, WPB, R, MINB, MODE>;
     // persistent grid: exactly the blocks that are resident at once
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep<DIR, NL, T, NT, R, MINB, MODE>, NT, bytes);
-    if (occ < 1) occ = 1;
-    const long long resident = (long long)nsm * occ;
-    const int grid = (int)(ntiles < resident ? ntiles : resident);
+    static const int resident = [&] {
+        int nsm = 148, occ = 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * WPB, bytes);
+        return nsm * (occ < 1 ? 1 : occ);
+    }();
+    a.seg_chunks = pick_chunks<DIR>(c.g, (long long)resident * WPB);
+    const long long blocks = (Cut<DIR, kLines>(c.g, a.seg_chunks).items() + WPB - 1) / WPB;
+    const int grid = (int)(blocks < resident ? blocks : resident);
     cudaEvent_t ev[2];
     timer_begin(c, ev);
-    k_sweep<DIR, NL, T, NT, R, MINB, MODE><<<grid, NT, bytes, c.stream>>>(a);
+    kern<<<grid, 32 * WPB, bytes, c.stream>>>(a);
     timer_end(c, ev);
     ++c.launches;
 }
 
-}  // namespace
-
-// Sweep tile shapes: x sweeps 1 line x 32 cells, y/z sweeps 2 lines x 16 cells.
-template <int DIR> struct SweepShape;
-template <> struct SweepShape<0> { static constexpr int NL = 1, T = 32; };
-template <> struct SweepShape<1> { static constexpr int NL = 2, T = 16; };
-template <> struct SweepShape<2> { static constexpr int NL = 2, T = 16; };
-
 template <int DIR>
-static int make_maps_dir(Ctx& c) {
-    using S = SweepShape<DIR>;
-    using TL = Tile<DIR, S::NL, S::T, double>;   // the TMA boxes do not depend on R
-    const Grid& g = c.g;
-    const uint64_t dims[4] = {(uint64_t)g.P0, (uint64_t)g.P1, (uint64_t)g.P2, 8};
-    const uint64_t strides[3] = {(uint64_t)g.pitch * 8, (uint64_t)g.pitch * g.P1 * 8, (uint64_t)g.fs * 8};
-    uint32_t bin[4], bout[4];
-    if (DIR == 0) { bin[0] = TL::C; bin[1] = S::NL; bin[2] = 1; bout[0] = TL::TO; bout[1] = S::NL; bout[2] = 1; }
-    else if (DIR == 1) { bin[0] = S::NL; bin[1] = TL::C; bin[2] = 1; bout[0] = S::NL; bout[1] = TL::TO; bout[2] = 1; }
-    else { bin[0] = S::NL; bin[1] = 1; bin[2] = TL::C; bout[0] = S::NL; bout[1] = 1; bout[2] = TL::TO; }
-    bin[3] = 8; bout[3] = 8;
+int make_maps_dir(Ctx& c) {
+    using M = WarpMem<DIR, kLines, double, 0>;   // the TMA boxes do not depend on R or MODE
     for (int b = 0; b < 6; ++b) {
-        int rc = encode_tensor_map_4d(&c.tm_in[b][DIR], c.qbuf[b], dims, strides, bin);
-        if (!rc) rc = encode_tensor_map_4d(&c.tm_out[b][DIR], c.qbuf[b], dims, strides, bout);
+        int rc = encode_sweep_maps(c.g, DIR, kLines, M::W, M::TO, c.qbuf[b], &c.tm_in[b][DIR], &c.tm_out[b][DIR]);
         if (rc) return rc;
     }
     return 0;
+}
+
+}  // namespace
+
+// The maps of one stage buffer: the raw tile (`cells` new cells of `lines`
+// lines, 8 variables) and the update operand (`op_cells`).
+int encode_sweep_maps(const Grid& g, int dir, int lines, int cells, int op_cells, const double* buf, CUtensorMap* in,
+                      CUtensorMap* out) {
+    const uint64_t dims[4] = {(uint64_t)g.P0, (uint64_t)g.P1, (uint64_t)g.P2, 8};
+    const uint64_t strides[3] = {(uint64_t)g.pitch * 8, (uint64_t)g.pitch * g.P1 * 8, (uint64_t)g.fs * 8};
+    uint32_t bin[4] = {1, 1, 1, 8}, bout[4] = {1, 1, 1, 8};
+    const int across = dir == 0 ? 1 : 0;
+    bin[dir] = (uint32_t)cells; bin[across] = (uint32_t)lines;
+    bout[dir] = (uint32_t)op_cells; bout[across] = (uint32_t)lines;
+    const int rc = encode_tensor_map_4d(in, buf, dims, strides, bin);
+    return rc ? rc : encode_tensor_map_4d(out, buf, dims, strides, bout);
 }
 
 int make_sweep_tensor_maps(Ctx& c) {
@@ -86,6 +95,7 @@ void launch_sweep(Ctx& c, int dir, const SweepArgs& a_in) {
     SweepArgs a = a_in;
     a.prof = c.prof;
     a.status = &c.dsc->status;
+    a.gam2 = (a.gam - 2.0) / (a.gam - 1.0);
     const int bin = buffer_of(c, a.qprev);
     const int bout = buffer_of(c, (a.mode == 0 || a.stage5) ? a.qout : a.q0);
     a.tm_in = c.tm_in[bin][dir];
@@ -118,25 +128,24 @@ void launch_sweep(Ctx& c, int dir, const SweepArgs& a_in) {
         a.route_prev = nullptr;
     }
     // instantiations: {fp64, mixed} x {plain, learned, guard-only}; label
-    // collection runs the FP64 method
-    // Blocks per SM (the launch bound that caps registers): six for the plain
-    // FP64 sweep (80 registers, one interface per thread in P3), seven for
-    // the learned one (72 registers), six for the plain mixed one (80
-    // registers, no spills); measured at 256^3 against 4/5 and 6/8 (FP64),
-    // 6 (learned) and 7 (plain mixed).
-#define HOW_SWEEP_CASES(D)                                                                              \
-    do {                                                                                                \
-        using S = SweepShape<D>;                                                                        \
-        if (mode == 3) { launch_one<D, S::NL, S::T, 128, double, 3, 3>(c, a); break; }                  \
-        if (mixed) {                                                                                    \
-            if (mode == 1) launch_one<D, S::NL, S::T, 128, float, 7, 1>(c, a);                          \
-            else if (mode == 2) launch_one<D, S::NL, S::T, 128, float, 5, 2>(c, a);                     \
-            else launch_one<D, S::NL, S::T, 128, float, 6, 0>(c, a);                                    \
-        } else {                                                                                        \
-            if (mode == 1) launch_one<D, S::NL, S::T, 128, double, 3, 1>(c, a);                         \
-            else if (mode == 2) launch_one<D, S::NL, S::T, 128, double, 3, 2>(c, a);                    \
-            else launch_one<D, S::NL, S::T, 128, double, 6, 0>(c, a);                                   \
-        }                                                                                               \
+    // collection runs the FP64 method.  Template arguments: warps per block
+    // and blocks per SM (the launch bound that caps registers).  FP64 at 8
+    // warps per SM (254 registers): 2.94 ms per 256^3 sweep, against 2.97 at
+    // 12 (168 registers, 144 bytes of spills) and 0.0674 against 0.0691 ms at
+    // 64^3.  Mixed at 12 (168 registers): 0.90 ms per 192^3 sweep, against
+    // 0.97 at the 128 registers of 16 warps, of which shared memory holds 12.
+#define HOW_SWEEP_CASES(D)                                              \
+    do {                                                                \
+        if (mode == 3) { launch_one<D, 4, double, 2, 3>(c, a); break; } \
+        if (mixed) {                                                    \
+            if (mode == 1) launch_one<D, 4, float, 3, 1>(c, a);         \
+            else if (mode == 2) launch_one<D, 4, float, 3, 2>(c, a);    \
+            else launch_one<D, 4, float, 3, 0>(c, a);                   \
+        } else {                                                        \
+            if (mode == 1) launch_one<D, 4, double, 2, 1>(c, a);        \
+            else if (mode == 2) launch_one<D, 4, double, 2, 2>(c, a);   \
+            else launch_one<D, 4, double, 2, 0>(c, a);                  \
+        }                                                               \
     } while (0)
     if (dir == 0) HOW_SWEEP_CASES(0);
     else if (dir == 1) HOW_SWEEP_CASES(1);
