@@ -151,7 +151,13 @@ static void run_stage(Ctx& c, int iw) {
 
 static void run_ssprk(Ctx& c) {
     nvtxRangePushA("ssprk");
+    const Grid& g = c.g;
+    const bool thin = (g.nx < 3 && c.p.bc[0] == HOW_BC_PERIODIC) || (g.ny < 3 && c.p.bc[1] == HOW_BC_PERIODIC) ||
+                      (g.nz < 3 && c.p.bc[2] == HOW_BC_PERIODIC);
+    c.one_pass_fill = !thin || c.axis_fill_steps == 0;
+    if (c.axis_fill_steps > 0) --c.axis_fill_steps;
     for (int iw = 1; iw <= 5; ++iw) run_stage(c, iw);
+    c.one_pass_fill = false;
     nvtxRangePop();
     // copy_stage(q, 0, 5); copy_bfield_to_stage0 (src/ssprk.cpp:1327-1328): swap
     std::swap(c.q[0], c.q[5]);
@@ -280,6 +286,7 @@ int how_set_state(how_ctx* c, int stage, const double* q) {
     const size_t n = 8 * ref_count(c->g);
     HOW_CUDA_CHECK(cudaMemcpyAsync(c->stage_buf, q, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     launch_ref_to_dev(*c, c->stage_buf, c->q[stage], 8);
+    c->axis_fill_steps = 2;
     if (stage == 0) c->have_state = true;
     c->route_valid = false;   // routing decisions are of the previous state
     return sync_and_status(*c);
@@ -300,6 +307,7 @@ int how_set_face_b(how_ctx* c, int stage, const double* bx, const double* by, co
     if (rc || (rc = check_stage(stage))) return rc;
     if (!bx || !by || !bz) { set_error("null face-B pointer"); return HOW_ERR_ARG; }
     const size_t n = ref_count(c->g);
+    c->axis_fill_steps = 2;
     const double* src[3] = {bx, by, bz};
     for (int k = 0; k < 3; ++k) {
         HOW_CUDA_CHECK(cudaMemcpyAsync(c->stage_buf + k * c->g.fs, src[k], n * sizeof(double),

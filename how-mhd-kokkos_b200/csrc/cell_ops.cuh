@@ -71,6 +71,74 @@ __device__ __forceinline__ int nb_off(const BCMap& m, int s, int d, int n, int p
     return m.on ? (bc_map(s + d, n, periodic) - s) * stride : d * stride;
 }
 
+// The three axes' fills in one pass.  An axis pass is a gather along that axis,
+// so x, then y, then z leave at (i, j, k) what was at (S_x(i), S_y(j), S_z(k))
+// before, with the index maps fill_source below.  For n >= 3 (and for an open
+// axis) every source is an active index: no cell read is written, and the
+// passes need no order.  A periodic axis of one or two cells also reads ghosts
+// that it overwrites (at(0) = at(1), at(1) = at(2) for n = 1): those cells are
+// moved by the thread of index 2, in increasing order, within its own column
+// of the other axes.  That column's ghosts hold what the passes would have put
+// there when the array has been filled before.
+__device__ __forceinline__ int fill_source(int s, int n, int periodic) {
+    if (s >= 3 && s <= n + 2) return s;
+    if (!periodic) return s < 3 ? 3 : n + 2;
+    if (s < 3) return n == 1 ? s + 1 : s + n;   // (n <= 2: may be a ghost)
+    return n == 1 ? 3 : n == 2 ? (s == 6 ? 4 : 3) : s - n;
+}
+
+// The extent of one such pass: ghost cells of the six z planes, of the six y
+// rows of the active planes, and of the six x columns of the active rows.
+__host__ __device__ __forceinline__ long long ghost_count(const Grid& g) {
+    return 6ll * g.P0 * g.P1 + 6ll * g.P0 * g.nz + 6ll * g.ny * g.nz;
+}
+
+// ghost cell t of every field (fields: array of nf base pointers)
+__device__ __forceinline__ void op_fill_ghost(const Grid& g, double* const* f, int nf, unsigned t, int px, int py,
+                                              int pz) {
+    int i, j, k;
+    const unsigned nzp = 6u * g.P0 * g.P1, nyp = 6u * g.P0 * g.nz;
+    if (t < nzp) {
+        const unsigned plane = (unsigned)g.P0 * g.P1, p = t / plane, r = t - p * plane;
+        j = (int)(r / g.P0); i = (int)(r - (unsigned)j * g.P0);
+        k = p < 3 ? (int)p : g.nz + (int)p;
+    } else if (t < nzp + nyp) {
+        t -= nzp;
+        const unsigned row = t / g.P0, c = row / 6u, p = row - c * 6u;
+        i = (int)(t - row * g.P0);
+        k = 3 + (int)c;
+        j = p < 3 ? (int)p : g.ny + (int)p;
+    } else {
+        t -= nzp + nyp;
+        const unsigned row = t / 6u, p = t - row * 6u;
+        k = 3 + (int)(row / g.ny); j = 3 + (int)(row % g.ny);
+        i = p < 3 ? (int)p : g.nx + (int)p;
+    }
+    // axes whose low ghosts read ghosts
+    const bool sx = px && g.nx < 3 && i < 3, sy = py && g.ny < 3 && j < 3, sz = pz && g.nz < 3 && k < 3;
+    if (!(sx || sy || sz)) {
+        const long long d = g.idx(i, j, k), s = g.idx(fill_source(i, g.nx, px), fill_source(j, g.ny, py),
+                                                      fill_source(k, g.nz, pz));
+        double v[12];
+#pragma unroll
+        for (int m = 0; m < 12; ++m) if (m < nf) v[m] = f[m][s];
+#pragma unroll
+        for (int m = 0; m < 12; ++m) if (m < nf) f[m][d] = v[m];
+        return;
+    }
+    if ((sx && i != 2) || (sy && j != 2) || (sz && k != 2)) return;
+    for (int c = sz ? 0 : k; c <= k; ++c)
+        for (int b = sy ? 0 : j; b <= j; ++b)
+            for (int a = sx ? 0 : i; a <= i; ++a) {
+                const int xs = fill_source(a, g.nx, px), ys = fill_source(b, g.ny, py), zs = fill_source(c, g.nz, pz);
+                // a ghost source: the other axes stay at this cell's index
+                const bool gx = sx && xs < 3, gy = sy && ys < 3, gz = sz && zs < 3;
+                const long long d = g.idx(a, b, c);
+                const long long s = gx || gy || gz ? g.idx(gx ? xs : a, gy ? ys : b, gz ? zs : c) : g.idx(xs, ys, zs);
+                for (int m = 0; m < nf; ++m) f[m][d] = f[m][s];
+            }
+}
+
 // columns of one field: (fast transverse extent, slow transverse extent)
 template <int AX>
 __host__ __device__ __forceinline__ void bound_plane(const Grid& g, int& ta, int& tb) {

@@ -184,6 +184,12 @@ struct Ctx {
     bool route_valid = false;
     long long route_age = 0;
     bool route_due = true;
+    // Ghost fills of the step in one launch per array set (k_fill_ghosts).  It
+    // relies on the arrays having been filled before when a periodic axis has
+    // one or two cells, so the two steps after a caller wrote a stage (which
+    // reach every buffer) fill axis by axis, as the standalone entry points do.
+    bool one_pass_fill = false;
+    int axis_fill_steps = 0;
     int wait_expire = 0;                  // failure-detection test hook (SweepArgs::wait_expire)
     // part of a domain decomposed into z slabs (how_group_*): the global z
     // index of local plane 3 minus 3, and which z ghost layers this context
