@@ -20,6 +20,8 @@ static TimerPool& pool(Ctx& c) {
     return pools.back().second;
 }
 
+bool timer_on(Ctx& c) { return pool(c).on; }
+
 void timer_begin(Ctx& c, cudaEvent_t* pair_out) {
     TimerPool& tp = pool(c);
     pair_out[0] = pair_out[1] = nullptr;
