@@ -20,21 +20,20 @@ constexpr ShapeDef kShapes[3][kEnsShapes] = {
     {{4, 2}, {4, 8}, {2, 2}},
     {{4, 2}, {4, 8}, {4, 4}},
 };
-constexpr int kWarps = 4, kBlocks = 2;   // warps per block, blocks per SM: as the single-domain FP64 sweep
+constexpr int kWarps = 12, kBlocks = 1;   // warps per block, blocks per SM: as the single-domain FP64 sweep
 
 template <int DIR, int NL>
 void launch_ens(SweepArgs a0, int chunks, cudaStream_t st, int dev) {
     constexpr int bytes = kWarps * WarpMem<DIR, NL, double, 0>::bytes + 128;
     const auto kern = k_sweep<DIR, NL, kWarps, double, kBlocks, 0, true>;
-    static const int resident = [&] {
-        int nsm = 148, occ = 0;
+    static const int nsm = [&] {   // one block per SM
+        int n = 148;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * kWarps, bytes);
-        return nsm * (occ < 1 ? 1 : occ);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n;
     }();
     a0.seg_chunks = chunks;
-    kern<<<resident, 32 * kWarps, bytes, st>>>(a0);
+    kern<<<nsm, 32 * kWarps, bytes, st>>>(a0);
 }
 
 template <int DIR>

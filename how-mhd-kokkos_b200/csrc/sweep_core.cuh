@@ -55,6 +55,7 @@
 #include "how_internal.cuh"
 #include "router.cuh"
 #include "tma.cuh"
+#include "tmem.cuh"
 
 #include <type_traits>
 
@@ -155,7 +156,8 @@ struct WarpMem {
     static constexpr int bU = bB + 8 * 3 * CB;                      // [4][NL] M, E of the last cell before
     static constexpr int bX = bU + 8 * 4 * NL;                      // [7][NL] interface flux before
     static constexpr int bBar = bX + 8 * 7 * NL;                    // 2 mbarriers: raw, operand
-    static constexpr int bD = align_up(bBar + 16, 16);              // [14][CD] differences of (F, q), R
+    static constexpr int bS = bBar + 16;                            // [32] the lanes' offsets (see spot)
+    static constexpr int bD = align_up(bS + 8 * 32, 16);              // [14][CD] differences of (F, q), R
     static constexpr int bL = align_up(bD + (int)sizeof(R) * 14 * CD, 16);   // [7][CL] |lambda|, R
     static constexpr int bC = align_up(bL + (int)sizeof(R) * 7 * CL, 16);    // [NCF][CL] FP32
     static constexpr int bytes = align_up(bC + 4 * NCF * CL, 128);
@@ -361,6 +363,41 @@ __device__ __forceinline__ void cell_values(const double* q, double gam, double 
     }
 }
 
+// N values of the working type per lane to tensor memory, and TIMES groups of N,
+// STEP values apart, from it
+template <int N> __device__ __forceinline__ void put_values(uint32_t at, const double* v) {
+    static_assert(N == 5, "");
+    uint32_t w[2 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) { w[2 * i] = (uint32_t)__double2loint(v[i]); w[2 * i + 1] = (uint32_t)__double2hiint(v[i]); }
+    tmem_store<8>(at, w);
+    tmem_store<2>(at + 8, w + 8);
+}
+template <int N> __device__ __forceinline__ void put_values(uint32_t at, const float* v) {
+    static_assert(N == 5, "");
+    uint32_t w[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = (uint32_t)__float_as_int(v[i]);
+    tmem_store<4>(at, w);
+    tmem_store<1>(at + 4, w + 4);
+}
+template <int N, int TIMES, int STEP> __device__ __forceinline__ void get_values(uint32_t at, double* v) {
+    uint32_t w[2 * N * TIMES];
+#pragma unroll
+    for (int i = 0; i < TIMES; ++i) tmem_load<2 * N>(at + 2 * STEP * i, w + 2 * N * i);
+    tmem_wait_loads<2 * N * TIMES>(w);
+#pragma unroll
+    for (int i = 0; i < N * TIMES; ++i) v[i] = __hiloint2double((int)w[2 * i + 1], (int)w[2 * i]);
+}
+template <int N, int TIMES, int STEP> __device__ __forceinline__ void get_values(uint32_t at, float* v) {
+    uint32_t w[N * TIMES];
+#pragma unroll
+    for (int i = 0; i < TIMES; ++i) tmem_load<N>(at + STEP * i, w + N * i);
+    tmem_wait_loads<N * TIMES>(w);
+#pragma unroll
+    for (int i = 0; i < N * TIMES; ++i) v[i] = __int_as_float((int)w[i]);
+}
+
 // The interface between the first two cells of the window at P (the lane's
 // column): eigen-system, projection, WENO5 of the seven fields and
 // back-projection.  out: the upwind correction to the left cell's flux.
@@ -373,8 +410,8 @@ struct FaceValues {
 };
 
 template <int NL, int CP, int CB, int CD, int CL, int MODE, typename R, typename Before>
-__device__ __forceinline__ void face_values(const double* sP, const double* sB, const R* sD, const R* sL, R gamR, R gam2,
-                                            FaceValues<R>& o, Before before_back) {
+__device__ __forceinline__ void face_values(const double* sP, const double* sB, const R* sD, const R* sL, uint32_t tm, R gamR,
+                                            R gam2, FaceValues<R>& o, Before before_back) {
     if constexpr (MODE == 3) o.departure = 0.0f;
     const R gam0 = R(1) - gamR;
     // eigen-system of the arithmetic mean of the two cells'
@@ -439,42 +476,50 @@ __device__ __forceinline__ void face_values(const double* sP, const double* sB, 
     };
     const R hn = R(0.5) * ics2;   // the rows' normalisation
     const R cen = -gam0 * ics2;
-    // Three pairs of fields, one loop body: fast (0, 6) with the
-    // entropy field, slow (2, 4), Alfven (1, 5).  Unrolled, the
-    // chunk's code no longer fits the instruction caches (0.5 ms
-    // of 3.8 per 256^3 sweep); and the differences are read once
-    // per pair, since two pairs' products do not fit 168 registers.
+    // Three pairs of fields: fast (0, 6), slow (2, 4), Alfven (1, 5), and the
+    // entropy field.  The differences are read once for the magnetosonic and
+    // entropy fields; their products (50 values a lane) wait in tensor memory
+    // for the loop over the pairs, whose two WENO fluxes are then the only copy
+    // of that code but one.  Held in registers the products leave room for 8
+    // warps per SM instead of 12, and unroll the loop past the instruction
+    // caches; formed again for each pair they cost 120 FP64 operations and 70
+    // shared-memory loads more.  The Alfven pair shares no product.
     R F0, F1, F2, F3, F4, F5, F6;
+    constexpr uint32_t RW = sizeof(R) / 4;   // columns per value
+    {
+        const R cef = hn * gam0 * af, cbf = hn * cs * as * sqr, cxf = hn * lf * af, ctf = -hn * as * ls * sgnB;
+        const R ces = hn * gam0 * as, cbs = -hn * cs * af * sqr, cxs = hn * ls * as, cts = hn * af * lf * sgnB;
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const R* D = sD + (7 * h) * CD + k * NL;
+                const R D0 = D[0], D1 = D[CD], D2 = D[2 * CD], D3 = D[3 * CD], D4 = D[4 * CD], D5 = D[5 * CD];
+                const R e = fm(-hvv, D0, fm(vx, D1, fm(vy, D2, fm(vz, D3, fm(By, D4, fm(Bz, D5, -D[6 * CD]))))));
+                const R b = fm(bty, D4, btz * D5);
+                const R x = fm(-vx, D0, D1);
+                const R t = fm(bty, D2, fm(btz, D3, -btv * D0));
+                const R fe = fm(cef, e, cbf * b), fo = fm(cxf, x, ctf * t);
+                const R se = fm(ces, e, cbs * b), so = fm(cxs, x, cts * t);
+                const R v[5] = {fe - fo, fe + fo, se - so, se + so, fm(cen, e, D0)};
+                put_values<5>(tm + (h * 5 + k) * 5 * RW, v);
+            }
+        tmem_wait_stores();
+    }
 #pragma unroll 1
     for (int pair = 0; pair < 3; ++pair) {
-        R mn[2][5], pl[2][5];
+        R v[20];
         if (pair < 2) {
-            const bool slow_pair = pair == 1;
-            const R a1 = slow_pair ? as : af, a2 = slow_pair ? af : as, l1 = slow_pair ? ls : lf,
-                    l2 = slow_pair ? lf : ls, tau = slow_pair ? R(-1) : R(1);
-            const R ce = hn * gam0 * a1, cb = tau * hn * cs * a2 * sqr, cx = hn * l1 * a1,
-                    ct = -tau * hn * a2 * l2 * sgnB;
-            R en[2][5];
+            // [difference][minus, plus] of the pair
+            R w[20];
+            get_values<2, 10, 5>(tm + pair * 2 * RW, w);
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int k = 0; k < 5; ++k) {
-                    const R* D = sD + (7 * h) * CD + k * NL;
-                    const R D0 = D[0], D1 = D[CD], D2 = D[2 * CD], D3 = D[3 * CD], D4 = D[4 * CD],
-                            D5 = D[5 * CD];
-                    const R e = fm(-hvv, D0, fm(vx, D1, fm(vy, D2, fm(vz, D3, fm(By, D4, fm(Bz, D5, -D[6 * CD]))))));
-                    const R b = fm(bty, D4, btz * D5);
-                    const R x = fm(-vx, D0, D1);
-                    const R t = fm(bty, D2, fm(btz, D3, -btv * D0));
-                    const R ev = fm(ce, e, cb * b), od = fm(cx, x, ct * t);
-                    mn[h][k] = ev - od;
-                    pl[h][k] = ev + od;
-                    en[h][k] = fm(cen, e, D0);
-                }
-            if (pair == 0) F3 = field(3, en[0], en[1]);
+                for (int k = 0; k < 5; ++k) { v[10 * h + k] = w[2 * (5 * h + k)]; v[10 * h + 5 + k] = w[2 * (5 * h + k) + 1]; }
         } else {
             const R cv = R(0.5) * fm(btz, vy, -(bty * vz)), cy = R(0.5) * bty, cz = R(0.5) * btz;
-            const R cb = sgnB * sqr, cby = cb * cy, cbz = cb * cz;
+            const R cm = sgnB * sqr, cby = cm * cy, cbz = cm * cz;
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -482,15 +527,20 @@ __device__ __forceinline__ void face_values(const double* sP, const double* sB, 
                     const R* D = sD + (7 * h) * CD + k * NL;
                     const R ev = fm(cv, D[0], fm(cy, D[3 * CD], -(cz * D[2 * CD])));
                     const R od = fm(cbz, D[4 * CD], -(cby * D[5 * CD]));
-                    mn[h][k] = ev - od;
-                    pl[h][k] = ev + od;
+                    v[10 * h + k] = ev - od;
+                    v[10 * h + 5 + k] = ev + od;
                 }
         }
         const int m = pair == 0 ? 0 : 3 - pair;   // 0, 2, 1
-        const R lo = field(m, mn[0], mn[1]), hi = field(6 - m, pl[0], pl[1]);
+        const R lo = field(m, v, v + 10), hi = field(6 - m, v + 5, v + 15);
         if (pair == 0) { F0 = lo; F6 = hi; }
         else if (pair == 1) { F2 = lo; F4 = hi; }
         else { F1 = lo; F5 = hi; }
+    }
+    {
+        R v[10];
+        get_values<1, 10, 5>(tm + 4 * RW, v);
+        F3 = field(3, v, v + 5);
     }
 
     before_back();
@@ -573,10 +623,35 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     double* sU = reinterpret_cast<double*>(sm + M::bU) + l;
     double* sX = reinterpret_cast<double*>(sm + M::bX) + l;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + M::bBar);
+    volatile long long* sSpot = reinterpret_cast<long long*>(sm + M::bS) + lane;
 
-    // one place of the march: an item's segment and the chunk in it (-1: the
-    // five cells before the first interface, no interface yet)
-    struct Place { long long item; const SweepArgs* a; int t1_0, t2, seg, fa, k, last; };
+    // tensor memory: a warp reaches lanes 32 (warp % 4) on, and the warps that
+    // share them take columns of their own.  (A kernel that allocates tensor
+    // memory runs one block per SM, so the block holds all of the SM's warps.)
+    static_assert(WPB % 4 == 0, "blocks of whole tensor memory lanes");
+    constexpr int kValues = 50, kPer = (kValues * (int)sizeof(R) / 4 + 3) / 4 * 4;   // columns per warp
+    constexpr int kUsed = WPB / 4 * kPer, kColumns = kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
+    static_assert(kUsed <= 512, "tensor memory has 512 columns");
+    __shared__ uint32_t s_tmem;
+    if (warp == 0) tmem_alloc<kColumns>(&s_tmem);
+    __syncthreads();
+    const uint32_t tm = s_tmem + ((uint32_t)(32 * (warp % 4)) << 16) + (uint32_t)(warp / 4 * kPer);
+
+    // One place of the march: a chunk (first interface fb) of an item's segment
+    // (last chunk's first interface fend, first owned interface lo; the chunk
+    // before the first, with the five cells before the first interface, has no
+    // interface yet).  FP64 at 12 warps keeps it in shared memory and reads it
+    // again where it is used: held across a chunk it takes 15 of 168 registers
+    // (256^3 sweep 3.05 ms with it, 2.54 without; the mixed method has them to
+    // spare, 0.85 against 0.89 ms at 192^3).
+    struct Place { int fb, fend, lo, t1_0, t2, item; const SweepArgs* a; };
+    constexpr bool FREE_REGS = sizeof(R) == 4 || WPB <= 8;
+    __shared__ Place s_place[FREE_REGS ? 1 : WPB];
+    Place r_place;
+    auto& here = [&]() -> std::conditional_t<FREE_REGS, Place&, volatile Place&> {
+        if constexpr (FREE_REGS) return r_place; else return s_place[warp];
+    }();
+    auto first_chunk = [](int lo, int fb) { return fb >= lo - CUT::ov; };   // an interface chunk
     auto member_of = [&](long long item) -> int {
         int lo = 0, hi = a0.ens_n - 1;   // last member whose first item is <= item
         while (lo < hi) {
@@ -585,48 +660,38 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
         }
         return lo;
     };
-    const int chunks = a0.seg_chunks;
-    long long nitems;
-    if constexpr (ENS) nitems = a0.ens_tile_start[a0.ens_n];
-    else nitems = CUT(a0.g, chunks).items();
-    const long long stride = (long long)gridDim.x * WPB;
+    // (a sweep has fewer than 2^31 items)
+    const int nitems = ENS ? (int)a0.ens_tile_start[a0.ens_n] : (int)CUT(a0.g, a0.seg_chunks).items();
     // the item's first place; items of members that are not stepping are skipped whole
-    auto enter = [&](long long item) -> Place {
-        Place p;
-        p.a = &a0;
-        long long li = item;
+    auto enter = [&](int item) -> Place {
+        const int chunks = a0.seg_chunks, stride = (int)gridDim.x * WPB;
+        Place p{0, 0, 0, 0, 0, item, &a0};
+        int li = item;
         if constexpr (ENS) {
             while (item < nitems) {
                 const int m = member_of(item);
                 if (a0.ens_active[m]) {
                     p.a = a0.ens_tab + ((long long)m * a0.ens_stride + a0.ens_off + a0.ens_par[m]);
-                    li = item - a0.ens_tile_start[m];
+                    li = item - (int)a0.ens_tile_start[m];
                     break;
                 }
-                const long long end = a0.ens_tile_start[m + 1];
+                const int end = (int)a0.ens_tile_start[m + 1];
                 item += (end - item + stride - 1) / stride * stride;
             }
+            p.item = item;
         }
-        p.item = item;
-        p.t1_0 = p.t2 = p.seg = p.fa = p.last = 0;
-        p.k = -1;
         if (item >= nitems) return p;
         const CUT c(p.a->g, chunks);
-        // line groups fastest: neighbouring warps work on neighbouring lines
-        // (a sweep has fewer than 2^31 items, so 32-bit divisions serve)
+        // line groups fastest: neighbouring lines are worked on at the same time
         const unsigned u = (unsigned)li, r = u / (unsigned)c.groups;
         p.t1_0 = CUT::line0 + NL * (int)(u - r * (unsigned)c.groups);
-        const unsigned sg = r / (unsigned)c.nt2;
-        p.t2 = 3 + (int)(r - sg * (unsigned)c.nt2);
-        p.seg = (int)sg;
-        p.fa = CUT::f0 + (int)sg * (chunks * W - CUT::ov);
-        const int all = (c.n - p.fa) / W;   // chunk of the last interface n
-        p.last = all < chunks - 1 ? all : chunks - 1;
+        const unsigned seg = r / (unsigned)c.nt2;
+        p.t2 = 3 + (int)(r - seg * (unsigned)c.nt2);
+        const int fa = CUT::f0 + (int)seg * (chunks * W - CUT::ov), all = (c.n - fa) / W;   // chunk of the last interface n
+        p.lo = seg == 0 ? 0 : fa + CUT::ov;
+        p.fb = fa - W;
+        p.fend = fa + (all < chunks - 1 ? all : chunks - 1) * W;
         return p;
-    };
-    auto after = [&](const Place& p) -> Place {
-        if (p.k < p.last) { Place q = p; ++q.k; return q; }
-        return enter(p.item + stride);
     };
 
     if (lane == 0) {
@@ -637,22 +702,21 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     __syncwarp();
     bool issued = true;            // lane 0's view
     unsigned par = 0u, pend = 0u;  // per barrier: phase parity, copy in flight (lane 0's view)
-    // TMA loads (lane 0): the new cells of place p (which == 0), or the update
+    // TMA loads (lane 0): the new cells of a place (which == 0), or the update
     // operand of its chunk (which == 1): cells fb+2 .. fb+W+1
-    auto issue = [&](const Place& p, int which) -> bool {
-        const int fb = p.fa + p.k * W;
+    auto issue = [&](int which, const SweepArgs* a, int fb, int t1_0, int t2) -> bool {
         const int along = which == 0 ? fb + 5 : DIR == 0 ? fb + 1 : fb + 2;
-        const int c0 = DIR == 0 ? along : p.t1_0;
-        const int c1 = DIR == 0 ? p.t1_0 : DIR == 1 ? along : p.t2;
-        const int c2 = DIR == 2 ? along : p.t2;
+        const int c0 = DIR == 0 ? along : t1_0;
+        const int c1 = DIR == 0 ? t1_0 : DIR == 1 ? along : t2;
+        const int c2 = DIR == 2 ? along : t2;
         if (c0 & 1) {   // never issue a misaligned tensor copy
-            atomicOr(p.a->status, HOW_STATUS_TMA_ALIGN);
+            atomicOr(a->status, HOW_STATUS_TMA_ALIGN);
             return false;
         }
         pend |= 1u << which;
         mbar_arrive_expect_tx(&bars[which], which == 0 ? M::raw_bytes : M::op_bytes);
-        tma_load_4d(sm + (which == 0 ? M::bRaw : M::bOp), which == 0 ? &p.a->tm_in : &p.a->tm_out, &bars[which], c0,
-                    c1, c2, 0);
+        tma_load_4d(sm + (which == 0 ? M::bRaw : M::bOp), which == 0 ? &a->tm_in : &a->tm_out, &bars[which], c0, c1, c2,
+                    0);
         return true;
     };
     // the lanes' tile waits are bounded (a failure-detection test can make
@@ -680,39 +744,58 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     const bool timed = a0.prof != nullptr && lane == 0;
     if (timed)
         for (int k = 0; k < 12; ++k) s_prof[warp][k] = 0ull;
-    unsigned tprev = (unsigned)clock();
+    __shared__ unsigned s_clock[WPB];
+    if (timed) s_clock[warp] = (unsigned)clock();
     auto mark = [&](int ph) {
-        if (timed) {
-            const unsigned now = (unsigned)clock();
-            s_prof[warp][ph] += now - tprev;
+        if (a0.prof != nullptr && lane == 0) {
+            s_prof[warp][ph] += (unsigned)clock() - s_clock[warp];
             if (ph == 10) ++s_prof[warp][11];   // chunks
-            tprev = (unsigned)clock();
+            s_clock[warp] = (unsigned)clock();
         }
     };
-    // a single domain's dt / d is one value for the whole launch
-    const double dtdl_launch = ENS ? 0.0 : *a0.dtdl;
     unsigned n_full = 0, n_cheap = 0;   // routed interfaces of this warp
 
-    Place p = enter((long long)blockIdx.x * WPB + warp);
-    if (lane == 0 && p.item < nitems) issued = issue(p, 0);
-    while (p.item < nitems) {
-        const SweepArgs& a = *p.a;
+    {
+        // (items go to all blocks before a block gets a second one)
+        const Place p = enter(warp * (int)gridDim.x + (int)blockIdx.x);
+        if constexpr (FREE_REGS) r_place = p;
+        else if (lane == 0) s_place[warp] = p;
+        if (lane == 0) {
+            if (p.item < nitems) issued = issue(0, p.a, p.fb, p.t1_0, p.t2);
+        }
+        __syncwarp();
+    }
+    while (here.item < nitems) {
+        const SweepArgs& a = ENS ? *here.a : a0;
         const Grid& g = a.g;
         const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
         const int nt1 = DIR == 0 ? g.ny : g.nx;
-        const int fb = p.fa + p.k * W, f = fb + j;   // the chunk's first interface, the lane's
-        const int t1 = p.t1_0 + l;
-        const bool line_ok = t1 >= 3 && t1 <= nt1 + 2;
-        const long long sstride = DIR == 0 ? 1ll : DIR == 1 ? (long long)g.pitch : (long long)g.pitch * g.P1;
-        const long long line = DIR == 0 ? g.idx(0, t1, p.t2) : DIR == 1 ? g.idx(t1, 0, p.t2) : g.idx(t1, p.t2, 0);
-        const long long at = line + (long long)(f + 2) * sstride;   // the face, and the cell left of it
-        // faces this segment owns: all from its second (the x sweep: third)
-        // interface on, and face 0
-        const bool owned = line_ok && f <= n && f >= (p.seg == 0 ? 0 : p.fa + CUT::ov);
         const double gam = a.gam, gm1 = gam - 1.0;
+        // where the lane is: its face, its line, and whether its segment owns
+        // the face (all from its second, in the x sweep third, interface on,
+        // and face 0)
+        struct Spot { int f, t1, t2; bool owned; };
+        auto spot = [&]() -> Spot {
+            Spot o;
+            o.f = here.fb + j; o.t1 = here.t1_0 + l; o.t2 = here.t2;
+            o.owned = o.t1 >= 3 && o.t1 <= nt1 + 2 && o.f <= n && o.f >= here.lo;
+            return o;
+        };
+        // an owned face's offset (and that of the cell left of it), for the
+        // stores: doubled, odd where the cell is the line's own (f >= 1); -1
+        // for a face the lane does not own
+        [[maybe_unused]] long long r_spot;
+        {
+            const Spot o = spot();
+            const long long at = DIR == 0 ? g.idx(o.f + 2, o.t1, o.t2)
+                               : DIR == 1 ? g.idx(o.t1, o.f + 2, o.t2) : g.idx(o.t1, o.t2, o.f + 2);
+            const long long code = o.owned ? 2 * at + (o.f >= 1 ? 1 : 0) : -1;
+            if constexpr (FREE_REGS) r_spot = code; else *sSpot = code;
+        }
+        auto spot_code = [&]() -> long long { if constexpr (FREE_REGS) return r_spot; else return *sSpot; };
 
         // -------------------------------------------------------------- load
-        if (!arrived(0)) return;   // results void; host sees the status
+        if (!arrived(0)) break;   // results void; host sees the status
         double q[8];
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
@@ -720,12 +803,22 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
             q[v] = DIR == 0 ? sRaw[(gv * NL + l) * W + j] : sRaw[gv * 32 + lane];
         }
         __syncwarp();   // every read of the raw tile, and of the window's new columns, is done
+        const bool faces = first_chunk(here.lo, here.fb);
         {
-            const Place nx = after(p);
-            if (lane == 0) {
-                fence_proxy_async_smem();
-                if (p.k >= 0) issued = issue(p, 1) && issued;
-                if (nx.item < nitems) issued = issue(nx, 0) && issued;
+            const int fb = here.fb, t1_0 = here.t1_0, t2 = here.t2;
+            if (fb < here.fend) {
+                if (lane == 0) {
+                    fence_proxy_async_smem();
+                    if (faces) issued = issue(1, &a, fb, t1_0, t2) && issued;
+                    issued = issue(0, &a, fb + W, t1_0, t2) && issued;
+                }
+            } else {
+                const Place nx = enter(here.item + (int)gridDim.x * WPB);
+                if (lane == 0) {
+                    fence_proxy_async_smem();
+                    if (faces) issued = issue(1, &a, fb, t1_0, t2) && issued;
+                    if (nx.item < nitems) issued = issue(0, nx.a, nx.fb, nx.t1_0, nx.t2) && issued;
+                }
             }
         }
         // MODE 1: the routing pass's decisions of the lane's face and its two
@@ -733,17 +826,16 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
         // valid while a feature moves by up to one cell)
         bool flagged = false;
         if constexpr (MODE == 1) {
-            if (p.k >= 0 && line_ok) {
-                const unsigned char* d = a.route_next + route_line(g, DIR, t1, p.t2) + (f + 2);
+            const Spot o = spot();
+            if (faces && o.t1 >= 3 && o.t1 <= nt1 + 2) {
+                const unsigned char* d = a.route_next + route_line(g, DIR, o.t1, o.t2) + (o.f + 2);
                 unsigned any = 0u;
 #pragma unroll
                 for (int s = -1; s <= 1; ++s)
-                    if (f + s >= 0 && f + s <= n) any |= d[s];
+                    if (o.f + s >= 0 && o.f + s <= n) any |= d[s];
                 flagged = any != 0u;
             }
         }
-        // this stage's dt / d (per member in an ensemble)
-        const double dtdl = ENS ? *a.dtdl : dtdl_launch;
         mark(0);
 
         // -------------------------------------------------------------- cell
@@ -789,7 +881,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
         }
         mark(1);
 
-        if (p.k >= 0) {
+        if (faces) {
             // ---------------------------------------------------------- face
             double fl[7];   // the interface's flux, rows rho, Mx, My, Mz, By, Bz, E of the line frame
             bool full = true;
@@ -800,20 +892,24 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
                 // the hard guard on this stage's state, whatever the stage
                 // the network's decisions were formed at
                 full = flagged || router_guard_rp(rr, pp, (float)a.rhomin, (float)a.pgmin, a.guard_jump, a.guard_floor);
-                const unsigned mf = __ballot_sync(ALL, owned && full), mc = __ballot_sync(ALL, owned && !full);
+                const Spot o = spot();
+                const unsigned mf = __ballot_sync(ALL, o.owned && full), mc = __ballot_sync(ALL, o.owned && !full);
                 n_full += __popc(mf);
                 n_cheap += __popc(mc);
                 if constexpr (MODE == 2) {
-                    if (owned) a.route_next[route_line(g, DIR, t1, p.t2) + (f + 2)] = (unsigned char)(full ? 1 : 0);
+                    if (o.owned) a.route_next[route_line(g, DIR, o.t1, o.t2) + (o.f + 2)] = (unsigned char)(full ? 1 : 0);
                 }
             }
             // the stage input of the cell left of the interface, which the
             // first sweep of a stage combines with the RK base (issued before
             // the back-projection, used at the update)
-            double prev[8];
+            // (with this stage's dt / d, per member in an ensemble)
+            double prev[8], dtdl;
             auto load_prev = [&] {
-                if (a.mode == 1 && owned && f >= 1) {
-                    const double* in = a.qprev + at;
+                dtdl = *a.dtdl;
+                const long long code = spot_code();
+                if (a.mode == 1 && (code & 1) && code > 0) {
+                    const double* in = a.qprev + (code >> 1);
 #pragma unroll
                     for (int gv = 0; gv < 8; ++gv, in += g.fs) prev[line_var(DIR, gv)] = *in;
                 }
@@ -825,7 +921,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
             // one of its faces does; a face keeps the result of its own
             if (!ROUTED || __any_sync(ALL, full)) {
                 FaceValues<R> fv;
-                face_values<NL, CP, CB, CD, CL, MODE>(sP, sB, sD, sL, R(gam), R(a.gam2), fv, load_prev);
+                face_values<NL, CP, CB, CD, CL, MODE>(sP, sB, sD, sL, tm, R(gam), R(a.gam2), fv, load_prev);
                 if constexpr (MODE == 3) lab_w = fv.departure;
 #pragma unroll
                 for (int r = 0; r < 7; ++r) {
@@ -876,13 +972,15 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
                 // the index of the tile of 32 faces, 1 line in x and 2 lines
                 // x 16 faces in y and z, so the sample does not alias with the
                 // grid nor depend on how the sweep is cut)
-                if (owned) {
-                    a.route_next[route_line(g, DIR, t1, p.t2) + (f + 2)] = 0;
+                const Spot o = spot();
+                if (o.owned) {
+                    const int f = o.f, t1 = o.t1;
+                    a.route_next[route_line(g, DIR, t1, o.t2) + (f + 2)] = 0;
                     constexpr int TL = DIR == 0 ? 1 : 2, TT = 32 / TL;
                     const int ntx = (n + TT - 1) / TT;
                     const int nty = DIR == 0 ? nt1 : (nt1 + 1 + TL - 1) / TL;
                     const int tx = f / TT < ntx ? f / TT : ntx - 1, ty = DIR == 0 ? t1 - 3 : (t1 - 2) / TL;
-                    const long long tile = ((long long)(p.t2 - 3) * nty + ty) * ntx + tx;
+                    const long long tile = ((long long)(o.t2 - 3) * nty + ty) * ntx + tx;
                     const unsigned long long hs = (unsigned long long)tile * 0x9E3779B97F4A7C15ull;
                     if ((unsigned int)(hs >> 32) % a.collect_every == 0u) {
                         StencilCell sc[6];
@@ -910,7 +1008,8 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
 
             // CT terms (src/ssprk.cpp:973-993): flux plus the mean of B_n v_t
             // over the two cells
-            if (owned) {
+            const long long code = spot_code();
+            if (code >= 0) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     const double* v = sB + c * CB + NL;       // v_t1 or v_t2 of cell f+2
@@ -924,7 +1023,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
                         // the reference's two-point form (-0, 9, 9, -0) / 18
                         avg = quot(fm(9.0, x1, 9.0 * x2), 18.0, 1.0 / 18.0);
                     }
-                    (c == 0 ? a.cta : a.ctb)[at] = fl[4 + c] + avg;
+                    (c == 0 ? a.cta : a.ctb)[code >> 1] = fl[4 + c] + avg;
                 }
             }
             mark(9);
@@ -936,18 +1035,18 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
                 const double up = __shfl_up_sync(ALL, fl[r], NL);
                 dfl[r] = fl[r] - (j == 0 ? sX[r * NL] : up);
             }
-            if (!arrived(1)) return;
+            if (!arrived(1)) break;
             // cell f+2, between this interface and the one before
-            if (owned && f >= 1) {
-                double* out = a.qout + at;
+            if (code >= 0 && (code & 1)) {
+                double* out = a.qout + (code >> 1);
 #pragma unroll
                 for (int gv = 0; gv < 8; ++gv, out += g.fs) {
                     const int v = line_var(DIR, gv);
                     const double cur = DIR == 0 ? sOp[(gv * NL + l) * M::TO + j + 1] : sOp[gv * 32 + lane];
-                    double o = a.mode == 1 ? fm(a.k3, prev[v], a.k1 * cur) : cur;
+                    double w = a.mode == 1 ? fm(a.k3, prev[v], a.k1 * cur) : cur;
                     // (the flux rows skip line variable 4, the normal B)
-                    if (v != 4) o = fm(-dtdl, dfl[v < 4 ? v : v - 1], o);
-                    if (v != 4 || a.mode != 0) *out = o;
+                    if (v != 4) w = fm(-dtdl, dfl[v < 4 ? v : v - 1], w);
+                    if (v != 4 || a.mode != 0) *out = w;
                 }
             }
             __syncwarp();   // every read of the operand tile and of sX is done
@@ -971,11 +1070,26 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
             }
             pf.store(sP - lane, lane); vb.store(sB - lane, lane); d.store(sD - lane, lane); e.store(sL - lane, lane);
         }
+        // the next place (in shared memory: read by all before lane 0 writes it,
+        // and written before the others read it)
+        if constexpr (FREE_REGS) {
+            if (here.fb < here.fend) here.fb += W;
+            else r_place = enter(here.item + (int)gridDim.x * WPB);
+        } else if (here.fb < here.fend) {
+            __syncwarp();
+            if (lane == 0) here.fb = here.fb + W;
+        } else {
+            const Place nx = enter(here.item + (int)gridDim.x * WPB);
+            __syncwarp();
+            if (lane == 0) s_place[warp] = nx;
+        }
+        __syncwarp();
         mark(10);
-        p = after(p);
     }
     if (timed)
         for (int k = 0; k < 12; ++k) atomicAdd(a0.prof + k, s_prof[warp][k]);
+    __syncthreads();   // every warp is done with its tensor memory
+    if (warp == 0) tmem_free<kColumns>(s_tmem);
     if constexpr (ROUTED) {
         if (lane == 0) {
             if (n_full) atomicAdd(&a0.route_count[0], (unsigned long long)n_full);

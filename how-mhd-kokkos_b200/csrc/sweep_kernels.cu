@@ -11,43 +11,60 @@ namespace {
 constexpr int kLines = 4;   // lines per warp: 32-byte rows in y and z
 
 // Length of the work items, in chunks: the one with the least time on the
-// busiest warp, rounds x (chunks + 1/4).  The quarter chunk stands for a
-// segment's first five cells, which have no interface yet.
+// busiest quarter of an SM, which holds `warps` warps at once.  A chunk takes
+// about 1 + w units of time with w warps beside one another (4.3k cycles alone
+// and 14k among three, FP64), and a segment's first five cells, which have no
+// interface yet, a quarter of a chunk.
+struct Plan { int chunks; long long each; };   // each: items per quarter of an SM
 template <int DIR>
-int pick_chunks(const Grid& g, long long warps) {
+Plan pick_chunks(const Grid& g, int nsm, int warps) {
     using CUT = Cut<DIR, kLines>;
     const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
     const int most = (n - CUT::f0) / CUT::W + 1;
-    int best = 1;
+    Plan best{1, 0};
     double best_t = 0.0;
     for (int s = 1; s <= most; ++s) {
-        const long long rounds = (CUT(g, s).items() + warps - 1) / warps;
-        const double t = (double)rounds * (s + 0.25);
-        if (s == 1 || t < best_t) { best = s; best_t = t; }
+        const long long each = (CUT(g, s).items() + 4 * nsm - 1) / (4 * nsm), rest = each % warps;
+        const double t = (double)(each / warps * (1 + warps) + (rest ? 1 + rest : 0)) * (s + 0.25);
+        if (s == 1 || t < best_t) { best = Plan{s, each}; best_t = t; }
     }
     return best;
 }
 
-template <int DIR, int WPB, typename R, int MINB, int MODE>
-void launch_one(Ctx& c, SweepArgs& a) {
-    constexpr int bytes = WPB * WarpMem<DIR, kLines, R, MODE>::bytes + 128;
-    const auto kern = k_sweep<DIR, kLines, WPB, R, MINB, MODE>;
-    // persistent grid: exactly the blocks that are resident at once
-    static const int resident = [&] {
-        int nsm = 148, occ = 0;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * WPB, bytes);
-        return nsm * (occ < 1 ? 1 : occ);
+int sm_count(const Ctx& c) {
+    static const int n = [&] {
+        int v = 148;
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, c.dev);
+        return v;
     }();
-    a.seg_chunks = pick_chunks<DIR>(c.g, (long long)resident * WPB);
-    const long long blocks = (Cut<DIR, kLines>(c.g, a.seg_chunks).items() + WPB - 1) / WPB;
-    const int grid = (int)(blocks < resident ? blocks : resident);
+    return n;
+}
+
+template <int DIR, int WPB, typename R, int MODE>
+void launch_plan(Ctx& c, SweepArgs& a, const Plan& plan) {
+    constexpr int bytes = WPB * WarpMem<DIR, kLines, R, MODE>::bytes + 128;
+    const auto kern = k_sweep<DIR, kLines, WPB, R, 1, MODE>;
+    static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    (void)set;
+    a.seg_chunks = plan.chunks;
+    // persistent grid: one block per SM (a kernel with tensor memory)
+    const long long items = Cut<DIR, kLines>(c.g, plan.chunks).items();
+    const int nsm = sm_count(c), grid = (int)(items < nsm ? items : nsm);
     cudaEvent_t ev[2];
     timer_begin(c, ev);
     kern<<<grid, 32 * WPB, bytes, c.stream>>>(a);
     timer_end(c, ev);
     ++c.launches;
+}
+
+// WPB warps per SM; SMALL (0: none) where no quarter of an SM gets more than
+// SMALL / 4 items
+template <int DIR, int WPB, int SMALL, typename R, int MODE>
+void launch_one(Ctx& c, SweepArgs& a) {
+    const Plan plan = pick_chunks<DIR>(c.g, sm_count(c), WPB / 4);
+    if constexpr (SMALL > 0)
+        if (plan.each <= SMALL / 4) return launch_plan<DIR, SMALL, R, MODE>(c, a, plan);
+    launch_plan<DIR, WPB, R, MODE>(c, a, plan);
 }
 
 template <int DIR>
@@ -128,24 +145,23 @@ void launch_sweep(Ctx& c, int dir, const SweepArgs& a_in) {
         a.route_prev = nullptr;
     }
     // instantiations: {fp64, mixed} x {plain, learned, guard-only}; label
-    // collection runs the FP64 method.  Template arguments: warps per block
-    // and blocks per SM (the launch bound that caps registers).  FP64 at 8
-    // warps per SM (254 registers): 2.94 ms per 256^3 sweep, against 2.97 at
-    // 12 (168 registers, 144 bytes of spills) and 0.0674 against 0.0691 ms at
-    // 64^3.  Mixed at 12 (168 registers): 0.90 ms per 192^3 sweep, against
-    // 0.97 at the 128 registers of 16 warps, of which shared memory holds 12.
-#define HOW_SWEEP_CASES(D)                                              \
-    do {                                                                \
-        if (mode == 3) { launch_one<D, 4, double, 2, 3>(c, a); break; } \
-        if (mixed) {                                                    \
-            if (mode == 1) launch_one<D, 4, float, 3, 1>(c, a);         \
-            else if (mode == 2) launch_one<D, 4, float, 3, 2>(c, a);    \
-            else launch_one<D, 4, float, 3, 0>(c, a);                   \
-        } else {                                                        \
-            if (mode == 1) launch_one<D, 4, double, 2, 1>(c, a);        \
-            else if (mode == 2) launch_one<D, 4, double, 2, 2>(c, a);   \
-            else launch_one<D, 4, double, 2, 0>(c, a);                  \
-        }                                                               \
+    // collection runs the FP64 method.  Template arguments: warps per SM, whose
+    // number caps the registers, and the warps of small domains.  FP64 at 12
+    // (168 registers): 2.54 ms per 256^3 sweep, against 2.64 at 8 (246); small
+    // domains at 8, whose chunk is shorter: 128^2 15.0 against 15.6 us.  Mixed at 12
+    // (168 registers): 0.85 ms per 192^3 sweep, against 1.01 at 8.
+#define HOW_SWEEP_CASES(D)                                                  \
+    do {                                                                    \
+        if (mode == 3) { launch_one<D, 8, 0, double, 3>(c, a); break; }     \
+        if (mixed) {                                                        \
+            if (mode == 1) launch_one<D, 12, 0, float, 1>(c, a);            \
+            else if (mode == 2) launch_one<D, 12, 0, float, 2>(c, a);       \
+            else launch_one<D, 12, 0, float, 0>(c, a);                      \
+        } else {                                                            \
+            if (mode == 1) launch_one<D, 8, 0, double, 1>(c, a);            \
+            else if (mode == 2) launch_one<D, 8, 0, double, 2>(c, a);       \
+            else launch_one<D, 12, 8, double, 0>(c, a);                     \
+        }                                                                   \
     } while (0)
     if (dir == 0) HOW_SWEEP_CASES(0);
     else if (dir == 1) HOW_SWEEP_CASES(1);
