@@ -87,43 +87,12 @@ __device__ __forceinline__ int fill_source(int s, int n, int periodic) {
     return n == 1 ? 3 : n == 2 ? (s == 6 ? 4 : 3) : s - n;
 }
 
-// The extent of one such pass: ghost cells of the six z planes, of the six y
-// rows of the active planes, and of the six x columns of the active rows.
-__host__ __device__ __forceinline__ long long ghost_count(const Grid& g) {
-    return 6ll * g.P0 * g.P1 + 6ll * g.P0 * g.nz + 6ll * g.ny * g.nz;
-}
-
-// ghost cell t of every field (fields: array of nf base pointers)
-__device__ __forceinline__ void op_fill_ghost(const Grid& g, double* const* f, int nf, unsigned t, int px, int py,
-                                              int pz) {
-    int i, j, k;
-    const unsigned nzp = 6u * g.P0 * g.P1, nyp = 6u * g.P0 * g.nz;
-    if (t < nzp) {
-        const unsigned plane = (unsigned)g.P0 * g.P1, p = t / plane, r = t - p * plane;
-        j = (int)(r / g.P0); i = (int)(r - (unsigned)j * g.P0);
-        k = p < 3 ? (int)p : g.nz + (int)p;
-    } else if (t < nzp + nyp) {
-        t -= nzp;
-        const unsigned row = t / g.P0, c = row / 6u, p = row - c * 6u;
-        i = (int)(t - row * g.P0);
-        k = 3 + (int)c;
-        j = p < 3 ? (int)p : g.ny + (int)p;
-    } else {
-        t -= nzp + nyp;
-        const unsigned row = t / 6u, p = t - row * 6u;
-        k = 3 + (int)(row / g.ny); j = 3 + (int)(row % g.ny);
-        i = p < 3 ? (int)p : g.nx + (int)p;
-    }
+// one ghost cell of a field
+__device__ __forceinline__ void op_fill_cell(const Grid& g, double* f, int i, int j, int k, int px, int py, int pz) {
     // axes whose low ghosts read ghosts
     const bool sx = px && g.nx < 3 && i < 3, sy = py && g.ny < 3 && j < 3, sz = pz && g.nz < 3 && k < 3;
     if (!(sx || sy || sz)) {
-        const long long d = g.idx(i, j, k), s = g.idx(fill_source(i, g.nx, px), fill_source(j, g.ny, py),
-                                                      fill_source(k, g.nz, pz));
-        double v[12];
-#pragma unroll
-        for (int m = 0; m < 12; ++m) if (m < nf) v[m] = f[m][s];
-#pragma unroll
-        for (int m = 0; m < 12; ++m) if (m < nf) f[m][d] = v[m];
+        f[g.idx(i, j, k)] = f[g.idx(fill_source(i, g.nx, px), fill_source(j, g.ny, py), fill_source(k, g.nz, pz))];
         return;
     }
     if ((sx && i != 2) || (sy && j != 2) || (sz && k != 2)) return;
@@ -133,10 +102,51 @@ __device__ __forceinline__ void op_fill_ghost(const Grid& g, double* const* f, i
                 const int xs = fill_source(a, g.nx, px), ys = fill_source(b, g.ny, py), zs = fill_source(c, g.nz, pz);
                 // a ghost source: the other axes stay at this cell's index
                 const bool gx = sx && xs < 3, gy = sy && ys < 3, gz = sz && zs < 3;
-                const long long d = g.idx(a, b, c);
-                const long long s = gx || gy || gz ? g.idx(gx ? xs : a, gy ? ys : b, gz ? zs : c) : g.idx(xs, ys, zs);
-                for (int m = 0; m < nf; ++m) f[m][d] = f[m][s];
+                f[g.idx(a, b, c)] = f[gx || gy || gz ? g.idx(gx ? xs : a, gy ? ys : b, gz ? zs : c) : g.idx(xs, ys, zs)];
             }
+}
+
+// One thread's part of such a pass over a field: the six z ghosts of a column
+// of the padded plane, the six y ghosts of an (x, active z) column, or one x
+// ghost of an active row.  A column's six loads go out before its stores, and
+// the lanes hold neighbouring i.
+__host__ __device__ __forceinline__ long long fill_parts(const Grid& g) {
+    return (long long)g.P0 * g.P1 + (long long)g.P0 * g.nz + 6ll * g.ny * g.nz;
+}
+__device__ __forceinline__ void op_fill_part(const Grid& g, double* f, unsigned t, int px, int py, int pz) {
+    const unsigned nzc = (unsigned)g.P0 * g.P1, nyc = (unsigned)g.P0 * g.nz;
+    if (t < nzc + nyc) {
+        const bool along_z = t < nzc;
+        if (!along_z) t -= nzc;
+        const int r = (int)(t / (unsigned)g.P0), i = (int)(t - (unsigned)r * g.P0);
+        const int n = along_z ? g.nz : g.ny, periodic = along_z ? pz : py;
+        const bool thin = (px && g.nx < 3 && i < 3) || (along_z && py && g.ny < 3 && r < 3);
+        if (thin) {
+            for (int m = 0; m < 6; ++m) {
+                const int s = m < 3 ? m : n + m;
+                if (along_z) op_fill_cell(g, f, i, r, s, px, py, pz);
+                else op_fill_cell(g, f, i, s, 3 + r, px, py, pz);
+            }
+            return;
+        }
+        const int xs = fill_source(i, g.nx, px), ys = along_z ? fill_source(r, g.ny, py) : 0;
+        const long long step = along_z ? (long long)g.pitch * g.P1 : (long long)g.pitch;
+        const long long own = along_z ? g.idx(i, r, 0) : g.idx(i, 0, 3 + r);
+        const long long from = along_z ? g.idx(xs, ys, 0) : g.idx(xs, 0, 3 + r);
+        double v[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int s = fill_source(m < 3 ? m : n + m, n, periodic);
+            v[m] = f[(s < 3 ? own : from) + s * step];   // (a ghost source: within this column)
+        }
+#pragma unroll
+        for (int m = 0; m < 6; ++m) f[own + (m < 3 ? m : n + m) * step] = v[m];
+        return;
+    }
+    t -= nzc + nyc;
+    const unsigned row = t / 6u, c = t - row * 6u;
+    const int k = (int)(row / (unsigned)g.ny), j = (int)(row - (unsigned)k * g.ny);
+    op_fill_cell(g, f, c < 3 ? (int)c : g.nx + (int)c, 3 + j, 3 + k, px, py, pz);
 }
 
 // columns of one field: (fast transverse extent, slow transverse extent)

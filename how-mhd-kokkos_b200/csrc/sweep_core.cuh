@@ -588,6 +588,11 @@ struct Cut {
     __host__ __device__ long long items() const { return (long long)groups * segs * nt2; }
 };
 
+template <bool FIRST, typename A, typename B>
+__device__ __forceinline__ auto& either(A& a, B& b) {
+    if constexpr (FIRST) return a; else return b;
+}
+
 // MODE 0: plain method.  1: learned routing (network + guard).  2: guard-only
 // routing (the ablation).  3: plain method that also records features and
 // nonlinear-weight labels of sampled tiles for training.
@@ -648,9 +653,8 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     constexpr bool FREE_REGS = sizeof(R) == 4 || WPB <= 8;
     __shared__ Place s_place[FREE_REGS ? 1 : WPB];
     Place r_place;
-    auto& here = [&]() -> std::conditional_t<FREE_REGS, Place&, volatile Place&> {
-        if constexpr (FREE_REGS) return r_place; else return s_place[warp];
-    }();
+    volatile Place& m_place = s_place[FREE_REGS ? 0 : warp];
+    auto& here = either<FREE_REGS>(r_place, m_place);
     auto first_chunk = [](int lo, int fb) { return fb >= lo - CUT::ov; };   // an interface chunk
     auto member_of = [&](long long item) -> int {
         int lo = 0, hi = a0.ens_n - 1;   // last member whose first item is <= item
