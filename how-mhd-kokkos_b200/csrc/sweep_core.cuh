@@ -197,9 +197,13 @@ struct MoveBack {
 };
 
 // One half of the WENO5-JS split (src/ssprk.cpp:883-937) from its four
-// arguments (twice the LLF-split differences; see weno_flux).  A common
-// factor of the three indicators cancels from the weights, so they are scaled
-// by 1/3 and eps with them: IS_k / 3 = 13/3 t^2 + t'^2.
+// arguments (twice the LLF-split differences; see weno_flux).  With t = a - b,
+// b - c, c - d the indicators are
+//   13 t^2 + 3 (a - 3 b)^2 = 16 t^2 - 12 b t + 12 b^2,    the same with (b + c),
+//   13 t^2 + 3 (3 c - d)^2 = 16 t^2 + 12 c t + 12 c^2,
+// and a common factor cancels from the weights, so they are formed as a twelfth
+// of that, eps with them, in eleven operations for the three (no term cancels
+// by more than a fifth: the least value over t is 13/16 b^2).
 //   w0 = P / D, w2 = 3 Q / D with e_k = (eps + IS_k)^2, P = e1 e2, Q = e0 e1,
 //   D = P + 6 e0 e2 + 3 Q;  X0, X1: the two second differences.
 template <typename R>
@@ -207,12 +211,10 @@ struct WenoHalf { R e0, e1, e2, X0, X1; };
 
 template <typename R>
 __device__ __forceinline__ WenoHalf<R> weno_half(R a, R b, R c, R d) {
-    const R K = R(13.0 / 3.0), eps = R(4.0e-10 / 3.0);
+    const R K = R(4.0 / 3.0), eps = R(4.0e-10 / 12.0);
     const R t0 = a - b, t2 = b - c, t4 = c - d;
-    const R t1 = fm(R(-3), b, a), t3 = b + c, t5 = fm(R(3), c, -d);
-    const R d0 = fm(t1, t1, fm(K * t0, t0, eps));
-    const R d1 = fm(t3, t3, fm(K * t2, t2, eps));
-    const R d2 = fm(t5, t5, fm(K * t4, t4, eps));
+    const R bb = fm(b, b, eps), cc = fm(c, c, eps);
+    const R d0 = fm(t0, fm(K, t0, -b), bb), d1 = fm(t2, fm(K, t2, -b), bb), d2 = fm(t4, fm(K, t4, c), cc);
     return WenoHalf<R>{d0 * d0, d1 * d1, d2 * d2, t0 - t2, t2 - t4};
 }
 
