@@ -130,6 +130,53 @@ __device__ __forceinline__ double larger(double a, double b) {
 }
 __device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
 
+// Two FP32 values that take the same operations: of a cell difference the
+// flux's and the state's part, of a field pair the minus and the plus field.
+// One packed instruction (add, sub, mul and fma.rn.f32x2) does both, rounded as
+// the two alone: the mixed sweep is bound by its instructions' issue (192^3
+// sweep 0.86 -> 0.76 ms).
+struct PairF { unsigned long long v; };
+
+__device__ __forceinline__ PairF make_pair(float a, float b) {
+    PairF r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ PairF both(float s) { return make_pair(s, s); }
+__device__ __forceinline__ PairF from_mem(float2 m) { return make_pair(m.x, m.y); }
+__device__ __forceinline__ void split(PairF p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+__device__ __forceinline__ PairF operator+(PairF x, PairF y) {
+    PairF r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ PairF operator-(PairF x, PairF y) {
+    PairF r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ PairF operator*(PairF x, PairF y) {
+    PairF r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ PairF fm(PairF x, PairF y, PairF z) {
+    PairF r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(x.v), "l"(y.v), "l"(z.v));
+    return r;
+}
+__device__ __forceinline__ PairF near_recip(PairF x) {
+    float a, b;
+    split(x, a, b);
+    return make_pair(near_recip(a), near_recip(b));
+}
+
+// The window's cell differences: FP64 keeps the rows of the flux's and the
+// state's differences apart (D + 7 rows), FP32 as pairs.
+template <typename R> struct Diff;
+template <> struct Diff<double> { using T = double; static constexpr int rows = 14; };
+template <> struct Diff<float> { using T = float2; static constexpr int rows = 7; };
+
 __host__ __device__ constexpr int align_up(int x, int a) { return (x + a - 1) / a * a; }
 
 // One warp's shared memory.  Window arrays are [row][column], a column per
@@ -157,7 +204,7 @@ struct WarpMem {
     static constexpr int bX = bU + 8 * 4 * NL;                      // [7][NL] interface flux before
     static constexpr int bBar = bX + 8 * 7 * NL;                    // 2 mbarriers: raw, operand
     static constexpr int bS = bBar + 16;                            // [32] the lanes' offsets (see spot)
-    static constexpr int bD = align_up(bS + 8 * 32, 16);              // [14][CD] differences of (F, q), R
+    static constexpr int bD = align_up(bS + 8 * 32, 16);              // [14][CD] differences of (F, q), R (Diff)
     static constexpr int bL = align_up(bD + (int)sizeof(R) * 14 * CD, 16);   // [7][CL] |lambda|, R
     static constexpr int bC = align_up(bL + (int)sizeof(R) * 7 * CL, 16);    // [NCF][CL] FP32
     static constexpr int bytes = align_up(bC + 4 * NCF * CL, 128);
@@ -206,16 +253,18 @@ struct MoveBack {
 // by more than a fifth: the least value over t is 13/16 b^2).
 //   w0 = P / D, w2 = 3 Q / D with e_k = (eps + IS_k)^2, P = e1 e2, Q = e0 e1,
 //   D = P + 6 e0 e2 + 3 Q;  X0, X1: the two second differences.
-template <typename R>
-struct WenoHalf { R e0, e1, e2, X0, X1; };
+// (V: a value or a pair of them; k: both() of a constant.  The differences are
+// taken with the signs that need no negation: X1m = -X1.)
+template <typename V>
+struct WenoHalf { V e0, e1, e2, X0, X1m; };
 
-template <typename R>
-__device__ __forceinline__ WenoHalf<R> weno_half(R a, R b, R c, R d) {
-    const R K = R(4.0 / 3.0), eps = R(4.0e-10 / 12.0);
-    const R t0 = a - b, t2 = b - c, t4 = c - d;
-    const R bb = fm(b, b, eps), cc = fm(c, c, eps);
-    const R d0 = fm(t0, fm(K, t0, -b), bb), d1 = fm(t2, fm(K, t2, -b), bb), d2 = fm(t4, fm(K, t4, c), cc);
-    return WenoHalf<R>{d0 * d0, d1 * d1, d2 * d2, t0 - t2, t2 - t4};
+template <typename V, typename K>
+__device__ __forceinline__ WenoHalf<V> weno_half(V a, V b, V c, V d, K k) {
+    const V g = k(4.0 / 3.0), eps = k(4.0e-10 / 12.0);
+    const V t0 = b - a, t2 = c - b, t4 = c - d;   // -t, -t, t above
+    const V bb = fm(b, b, eps), cc = fm(c, c, eps);
+    const V d0 = fm(t0, fm(g, t0, b), bb), d1 = fm(t2, fm(g, t2, b), bb), d2 = fm(t4, fm(g, t4, c), cc);
+    return WenoHalf<V>{d0 * d0, d1 * d1, d2 * d2, t2 - t0, t2 + t4};
 }
 
 // Characteristic WENO5-JS/LLF flux of one field (src/ssprk.cpp:883-937) from
@@ -236,15 +285,16 @@ __device__ __forceinline__ WenoHalf<R> weno_half(R a, R b, R c, R d) {
 //    products of e_k would underflow) with fast reciprocals.
 template <bool DEV>
 __device__ __forceinline__ double weno_flux(const double* f, const double* q, double amx, double* dev) {
+    auto k = [](double c) { return c; };
     const WenoHalf<double> p = weno_half(fm(amx, q[0], f[0]), fm(amx, q[1], f[1]), fm(amx, q[2], f[2]),
-                                         fm(amx, q[3], f[3]));
+                                         fm(amx, q[3], f[3]), k);
     const WenoHalf<double> m = weno_half(fm(-amx, q[4], f[4]), fm(-amx, q[3], f[3]), fm(-amx, q[2], f[2]),
-                                         fm(-amx, q[1], f[1]));
+                                         fm(-amx, q[1], f[1]), k);
     const double Pp = p.e1 * p.e2, Qp = p.e0 * p.e1, Dp = fm(6.0, p.e0 * p.e2, fm(3.0, Qp, Pp));
     const double Pm = m.e1 * m.e2, Qm = m.e0 * m.e1, Dm = fm(6.0, m.e0 * m.e2, fm(3.0, Qm, Pm));
     // (the weights before their products with X: P X would overflow first)
     const double ip = near_recip(Dp), im = near_recip(Dm);
-    const double wp = fm(1.5, (Qp * ip) * p.X1, (Pp * ip) * p.X0), wm = fm(1.5, (Qm * im) * m.X1, (Pm * im) * m.X0);
+    const double wp = fm(-1.5, (Qp * ip) * p.X1m, (Pp * ip) * p.X0), wm = fm(-1.5, (Qm * im) * m.X1m, (Pm * im) * m.X0);
     if constexpr (DEV) {
         // largest departure of the nonlinear weights from the linear (0.1, 0.6, 0.3)
         const double w0p = Pp / Dp, w2p = 3.0 * Qp / Dp, w0m = Pm / Dm, w2m = 3.0 * Qm / Dm;
@@ -254,23 +304,24 @@ __device__ __forceinline__ double weno_flux(const double* f, const double* q, do
         *dev = fmax(d, fabs(1.0 - w0m - w2m - 0.6));
     }
     const double c = fm(6.0, f[2], f[1]) - f[3];
-    return fm(1.0 / 6.0, wm - wp, fm(1.0 / 12.0, c, (1.0 / 24.0) * (p.X1 - m.X1)));
+    return fm(1.0 / 6.0, wm - wp, fm(1.0 / 12.0, c, (1.0 / 24.0) * (m.X1m - p.X1m)));
 }
 
-template <bool DEV>
-__device__ __forceinline__ float weno_flux(const float* f, const float* q, float amx, float*) {
-    static_assert(!DEV, "labels are recorded by the FP64 method");
-    const WenoHalf<float> p = weno_half(fm(amx, q[0], f[0]), fm(amx, q[1], f[1]), fm(amx, q[2], f[2]),
-                                        fm(amx, q[3], f[3]));
-    const WenoHalf<float> m = weno_half(fm(-amx, q[4], f[4]), fm(-amx, q[3], f[3]), fm(-amx, q[2], f[2]),
-                                        fm(-amx, q[1], f[1]));
-    auto part = [](const WenoHalf<float>& h) {
-        const float a0 = near_recip(h.e0), a1 = 6.0f * near_recip(h.e1), a2 = 3.0f * near_recip(h.e2);
-        const float is = near_recip(a0 + a1 + a2);
-        return fm((a0 * is) * h.X0, 2.0f, fm(a2, is, -0.5f) * h.X1);
+// FP32, of one field (V = float) or two side by side (V = PairF)
+template <typename V, typename K>
+__device__ __forceinline__ V weno_flux32(const V* f, const V* q, V amx, V minus_amx, K k) {
+    const WenoHalf<V> p = weno_half(fm(amx, q[0], f[0]), fm(amx, q[1], f[1]), fm(amx, q[2], f[2]),
+                                    fm(amx, q[3], f[3]), k);
+    const WenoHalf<V> m = weno_half(fm(minus_amx, q[4], f[4]), fm(minus_amx, q[3], f[3]), fm(minus_amx, q[2], f[2]),
+                                    fm(minus_amx, q[1], f[1]), k);
+    // twelve times a half's weighted second differences, 2 w0 X0 + (w2 - 1/2) X1
+    auto part = [&](const WenoHalf<V>& h) {
+        const V a0 = near_recip(h.e0), a1 = k(6.0) * near_recip(h.e1), a2 = k(-3.0) * near_recip(h.e2);
+        const V is = near_recip(a0 + a1 - a2);
+        return fm((a0 * is) * h.X0, k(2.0), fm(a2, is, k(0.5)) * h.X1m);
     };
-    const float c = fm(6.0f, f[2], f[1]) - f[3];
-    return (1.0f / 12.0f) * (c - part(p) + part(m));
+    const V c = fm(k(6.0), f[2], f[1]) - f[3];
+    return k(1.0 / 12.0) * (c - part(p) + part(m));
 }
 
 // Component-wise fifth-order upwind flux with the linear weights
@@ -365,23 +416,21 @@ __device__ __forceinline__ void cell_values(const double* q, double gam, double 
     }
 }
 
-// N values of the working type per lane to tensor memory, and TIMES groups of N,
-// STEP values apart, from it
-template <int N> __device__ __forceinline__ void put_values(uint32_t at, const double* v) {
-    static_assert(N == 5, "");
-    uint32_t w[2 * N];
+// Values per lane to tensor memory, and TIMES groups of N, STEP values apart,
+// from it
+__device__ __forceinline__ void put_five(uint32_t at, const double* v) {
+    uint32_t w[10];
 #pragma unroll
-    for (int i = 0; i < N; ++i) { w[2 * i] = (uint32_t)__double2loint(v[i]); w[2 * i + 1] = (uint32_t)__double2hiint(v[i]); }
+    for (int i = 0; i < 5; ++i) { w[2 * i] = (uint32_t)__double2loint(v[i]); w[2 * i + 1] = (uint32_t)__double2hiint(v[i]); }
     tmem_store<8>(at, w);
     tmem_store<2>(at + 8, w + 8);
 }
-template <int N> __device__ __forceinline__ void put_values(uint32_t at, const float* v) {
-    static_assert(N == 5, "");
-    uint32_t w[N];
+__device__ __forceinline__ void put_ten(uint32_t at, const float* v) {
+    uint32_t w[10];
 #pragma unroll
-    for (int i = 0; i < N; ++i) w[i] = (uint32_t)__float_as_int(v[i]);
-    tmem_store<4>(at, w);
-    tmem_store<1>(at + 4, w + 4);
+    for (int i = 0; i < 10; ++i) w[i] = (uint32_t)__float_as_int(v[i]);
+    tmem_store<8>(at, w);
+    tmem_store<2>(at + 8, w + 8);
 }
 template <int N, int TIMES, int STEP> __device__ __forceinline__ void get_values(uint32_t at, double* v) {
     uint32_t w[2 * N * TIMES];
@@ -412,7 +461,8 @@ struct FaceValues {
 };
 
 template <int NL, int CP, int CB, int CD, int CL, int MODE, typename R, typename Before>
-__device__ __forceinline__ void face_values(const double* sP, const double* sB, const R* sD, const R* sL, uint32_t tm, R gamR,
+__device__ __forceinline__ void face_values(const double* sP, const double* sB, const typename Diff<R>::T* sD, const R* sL,
+                                            uint32_t tm, R gamR,
                                             R gam2, FaceValues<R>& o, Before before_back) {
     if constexpr (MODE == 3) o.departure = 0.0f;
     const R gam0 = R(1) - gamR;
@@ -466,15 +516,12 @@ __device__ __forceinline__ void face_values(const double* sP, const double* sB, 
     // (The reference turns the fast or slow rows and columns by
     // sgn(B_t), src/ssprk.cpp:789-818; the field's flux is odd in
     // its row, so the sign cancels exactly from row and column.)
-    auto field = [&](int m, const R* pf, const R* pq) -> R {
+    auto speed = [&](int m) -> R {   // the stencil's largest |lambda_m|
         const R* sm = sL + m * CL;
         R amx = sm[0];
 #pragma unroll
         for (int k = 1; k < 6; ++k) amx = larger(amx, sm[k * NL]);
-        R d = R(0);
-        const R r = weno_flux<MODE == 3>(pf, pq, amx, &d);
-        if constexpr (MODE == 3) o.departure = fmaxf(o.departure, (float)d);
-        return r;
+        return amx;
     };
     const R hn = R(0.5) * ics2;   // the rows' normalisation
     const R cen = -gam0 * ics2;
@@ -487,62 +534,137 @@ __device__ __forceinline__ void face_values(const double* sP, const double* sB, 
     // caches; formed again for each pair they cost 120 FP64 operations and 70
     // shared-memory loads more.  The Alfven pair shares no product.
     R F0, F1, F2, F3, F4, F5, F6;
-    constexpr uint32_t RW = sizeof(R) / 4;   // columns per value
     {
-        const R cef = hn * gam0 * af, cbf = hn * cs * as * sqr, cxf = hn * lf * af, ctf = -hn * as * ls * sgnB;
-        const R ces = hn * gam0 * as, cbs = -hn * cs * af * sqr, cxs = hn * ls * as, cts = hn * af * lf * sgnB;
+        if constexpr (std::is_same<R, double>::value) {
+            const double cef = hn * gam0 * af, cbf = hn * cs * as * sqr, cxf = hn * lf * af, ctf = -hn * as * ls * sgnB;
+            const double ces = hn * gam0 * as, cbs = -hn * cs * af * sqr, cxs = hn * ls * as, cts = hn * af * lf * sgnB;
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < 2; ++h)   // fluxes, states
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const double* D = sD + (7 * h) * CD + k * NL;
+                    const double D0 = D[0], D1 = D[CD], D2 = D[2 * CD], D3 = D[3 * CD], D4 = D[4 * CD], D5 = D[5 * CD];
+                    const double e = fm(-hvv, D0, fm(vx, D1, fm(vy, D2, fm(vz, D3, fm(By, D4, fm(Bz, D5, -D[6 * CD]))))));
+                    const double b = fm(bty, D4, btz * D5);
+                    const double x = fm(-vx, D0, D1);
+                    const double t = fm(bty, D2, fm(btz, D3, -btv * D0));
+                    const double fe = fm(cef, e, cbf * b), fo = fm(cxf, x, ctf * t);
+                    const double se = fm(ces, e, cbs * b), so = fm(cxs, x, cts * t);
+                    const double v[5] = {fe - fo, fe + fo, se - so, se + so, fm(cen, e, D0)};
+                    put_five(tm + (h * 5 + k) * 10, v);
+                }
+        } else {
+            using P = PairF;
+            const P cef = both(-hn * gam0 * af), cbf = both(hn * cs * as * sqr), cxf = both(hn * lf * af),
+                    ctf = both(-hn * as * ls * sgnB);
+            const P ces = both(-hn * gam0 * as), cbs = both(-hn * cs * af * sqr), cxs = both(hn * ls * as),
+                    cts = both(hn * af * lf * sgnB);
+            const P cen_ = both(-cen), h2 = both(hvv), nvx = both(-vx), nvy = both(-vy), nvz = both(-vz), nBy = both(-By),
+                    nBz = both(-Bz), by = both(bty), bz = both(btz), nbv = both(-btv);
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                const R* D = sD + (7 * h) * CD + k * NL;
-                const R D0 = D[0], D1 = D[CD], D2 = D[2 * CD], D3 = D[3 * CD], D4 = D[4 * CD], D5 = D[5 * CD];
-                const R e = fm(-hvv, D0, fm(vx, D1, fm(vy, D2, fm(vz, D3, fm(By, D4, fm(Bz, D5, -D[6 * CD]))))));
-                const R b = fm(bty, D4, btz * D5);
-                const R x = fm(-vx, D0, D1);
-                const R t = fm(bty, D2, fm(btz, D3, -btv * D0));
-                const R fe = fm(cef, e, cbf * b), fo = fm(cxf, x, ctf * t);
-                const R se = fm(ces, e, cbs * b), so = fm(cxs, x, cts * t);
-                const R v[5] = {fe - fo, fe + fo, se - so, se + so, fm(cen, e, D0)};
-                put_values<5>(tm + (h * 5 + k) * 5 * RW, v);
+                const auto* D = sD + k * NL;
+                const P D0 = from_mem(D[0]), D1 = from_mem(D[CD]), D2 = from_mem(D[2 * CD]), D3 = from_mem(D[3 * CD]),
+                        D4 = from_mem(D[4 * CD]), D5 = from_mem(D[5 * CD]), D6 = from_mem(D[6 * CD]);
+                const P ne = fm(h2, D0, fm(nvx, D1, fm(nvy, D2, fm(nvz, D3, fm(nBy, D4, fm(nBz, D5, D6))))));   // -e
+                const P b = fm(by, D4, bz * D5);
+                const P x = fm(nvx, D0, D1);
+                const P t = fm(by, D2, fm(bz, D3, nbv * D0));
+                R v[10], ef, eq, of, oq;   // per pair: flux minus, plus, state minus, plus; then the entropy field's
+                split(fm(cef, ne, cbf * b), ef, eq);
+                split(fm(cxf, x, ctf * t), of, oq);
+                v[0] = ef - of; v[1] = ef + of; v[2] = eq - oq; v[3] = eq + oq;
+                split(fm(ces, ne, cbs * b), ef, eq);
+                split(fm(cxs, x, cts * t), of, oq);
+                v[4] = ef - of; v[5] = ef + of; v[6] = eq - oq; v[7] = eq + oq;
+                split(fm(cen_, ne, D0), v[8], v[9]);
+                put_ten(tm + k * 10, v);
             }
+        }
         tmem_wait_stores();
     }
 #pragma unroll 1
     for (int pair = 0; pair < 3; ++pair) {
-        R v[20];
+        R w[20];   // per difference: flux minus, plus, state minus, plus
         if (pair < 2) {
-            // [difference][minus, plus] of the pair
-            R w[20];
-            get_values<2, 10, 5>(tm + pair * 2 * RW, w);
+            if constexpr (std::is_same<R, double>::value) {
+                double v[20];   // [flux, state][difference][minus, plus]
+                get_values<2, 10, 5>(tm + pair * 4, v);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int k = 0; k < 5; ++k) { v[10 * h + k] = w[2 * (5 * h + k)]; v[10 * h + 5 + k] = w[2 * (5 * h + k) + 1]; }
-        } else {
-            const R cv = R(0.5) * fm(btz, vy, -(bty * vz)), cy = R(0.5) * bty, cz = R(0.5) * btz;
-            const R cm = sgnB * sqr, cby = cm * cy, cbz = cm * cz;
+                for (int k = 0; k < 5; ++k) {
+                    w[4 * k] = v[2 * k]; w[4 * k + 1] = v[2 * k + 1];
+                    w[4 * k + 2] = v[10 + 2 * k]; w[4 * k + 3] = v[11 + 2 * k];
+                }
+            } else {
+                get_values<4, 5, 10>(tm + pair * 4, w);
+            }
+        } else if constexpr (std::is_same<R, double>::value) {
+            const double cv = 0.5 * fm(btz, vy, -(bty * vz)), cy = 0.5 * bty, cz = 0.5 * btz;
+            const double cm = sgnB * sqr, cby = cm * cy, cbz = cm * cz;
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
-                    const R* D = sD + (7 * h) * CD + k * NL;
-                    const R ev = fm(cv, D[0], fm(cy, D[3 * CD], -(cz * D[2 * CD])));
-                    const R od = fm(cbz, D[4 * CD], -(cby * D[5 * CD]));
-                    v[10 * h + k] = ev - od;
-                    v[10 * h + 5 + k] = ev + od;
+                    const double* D = sD + (7 * h) * CD + k * NL;
+                    const double ev = fm(cv, D[0], fm(cy, D[3 * CD], -(cz * D[2 * CD])));
+                    const double od = fm(cbz, D[4 * CD], -(cby * D[5 * CD]));
+                    w[4 * k + 2 * h] = ev - od;
+                    w[4 * k + 2 * h + 1] = ev + od;
                 }
+        } else {
+            using P = PairF;
+            const R cz = R(0.5) * btz, cm = sgnB * sqr;
+            const P cv = both(R(0.5) * fm(btz, vy, -(bty * vz))), cy = both(R(0.5) * bty), ncz = both(-cz);
+            const P cbz = both(cm * cz), ncby = both(-cm * (R(0.5) * bty));
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const auto* D = sD + k * NL;
+                const P ev = fm(cv, from_mem(D[0]), fm(cy, from_mem(D[3 * CD]), ncz * from_mem(D[2 * CD])));
+                const P od = fm(cbz, from_mem(D[4 * CD]), ncby * from_mem(D[5 * CD]));
+                R ef, eq, of, oq;
+                split(ev, ef, eq);
+                split(od, of, oq);
+                w[4 * k] = ef - of; w[4 * k + 1] = ef + of; w[4 * k + 2] = eq - oq; w[4 * k + 3] = eq + oq;
+            }
         }
         const int m = pair == 0 ? 0 : 3 - pair;   // 0, 2, 1
-        const R lo = field(m, v, v + 10), hi = field(6 - m, v + 5, v + 15);
+        R lo, hi;
+        if constexpr (std::is_same<R, double>::value) {
+            double f[5], q[5], d = 0.0;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) { f[k] = w[4 * k]; q[k] = w[4 * k + 2]; }
+            lo = weno_flux<MODE == 3>(f, q, speed(m), &d);
+            if constexpr (MODE == 3) o.departure = fmaxf(o.departure, (float)d);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) { f[k] = w[4 * k + 1]; q[k] = w[4 * k + 3]; }
+            hi = weno_flux<MODE == 3>(f, q, speed(6 - m), &d);
+            if constexpr (MODE == 3) o.departure = fmaxf(o.departure, (float)d);
+        } else {
+            PairF f[5], q[5];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) { f[k] = make_pair(w[4 * k], w[4 * k + 1]); q[k] = make_pair(w[4 * k + 2], w[4 * k + 3]); }
+            const float s0 = speed(m), s1 = speed(6 - m);
+            split(weno_flux32(f, q, make_pair(s0, s1), make_pair(-s0, -s1), [](double c) { return both((float)c); }), lo, hi);
+        }
         if (pair == 0) { F0 = lo; F6 = hi; }
         else if (pair == 1) { F2 = lo; F4 = hi; }
         else { F1 = lo; F5 = hi; }
     }
     {
-        R v[10];
-        get_values<1, 10, 5>(tm + 4 * RW, v);
-        F3 = field(3, v, v + 5);
+        R w[10];
+        const R s = speed(3);
+        if constexpr (std::is_same<R, double>::value) {
+            double d = 0.0;
+            get_values<1, 10, 5>(tm + 8, w);
+            F3 = weno_flux<MODE == 3>(w, w + 5, s, &d);
+            if constexpr (MODE == 3) o.departure = fmaxf(o.departure, (float)d);
+        } else {
+            float f[5], q[5];
+            get_values<2, 5, 10>(tm + 8, w);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) { f[k] = w[2 * k]; q[k] = w[2 * k + 1]; }
+            F3 = weno_flux32(f, q, s, -s, [](double c) { return (float)c; });
+        }
     }
 
     before_back();
@@ -624,7 +746,8 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     double* sP = reinterpret_cast<double*>(sm + M::bP) + lane;
     double* sB = reinterpret_cast<double*>(sm + M::bB) + lane;
     double* sF = reinterpret_cast<double*>(sm + M::bF) + lane;
-    R* sD = reinterpret_cast<R*>(sm + M::bD) + lane;
+    using DT = typename Diff<R>::T;
+    DT* sD = reinterpret_cast<DT*>(sm + M::bD) + lane;
     R* sL = reinterpret_cast<R*>(sm + M::bL) + lane;
     float* sC = reinterpret_cast<float*>(sm + M::bC) + lane;
     double* sU = reinterpret_cast<double*>(sm + M::bU) + l;
@@ -643,6 +766,12 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     if (warp == 0) tmem_alloc<kColumns>(&s_tmem);
     __syncthreads();
     const uint32_t tm = s_tmem + ((uint32_t)(32 * (warp % 4)) << 16) + (uint32_t)(warp / 4 * kPer);
+
+    // component r's k-th difference of the lane's stencil, flux and state
+    [[maybe_unused]] auto diff_at = [&](int r, int k, R& f, R& q) {
+        if constexpr (std::is_same<R, double>::value) { f = sD[r * CD + k * NL]; q = sD[(7 + r) * CD + k * NL]; }
+        else { const float2 d = sD[r * CD + k * NL]; f = d.x; q = d.y; }
+    };
 
     // One place of the march: a chunk (first interface fb) of an item's segment
     // (last chunk's first interface fend, first owned interface lo; the chunk
@@ -878,7 +1007,11 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
             const double now[14] = {cv.F[0], cv.F[1], cv.F[2], cv.F[3], cv.F[4], cv.F[5], cv.F[6],
                                     cv.rho, q[1], q[2], q[3], By, Bz, cv.EE};
 #pragma unroll
-            for (int v = 0; v < 14; ++v) sD[v * CD + nD] = R(now[v] - before[v]);
+            for (int v = 0; v < 7; ++v) {
+                const R d = R(now[v] - before[v]), e = R(now[7 + v] - before[7 + v]);
+                if constexpr (std::is_same<R, double>::value) { sD[v * CD + nD] = d; sD[(7 + v) * CD + nD] = e; }
+                else sD[v * CD + nD] = make_float2(d, e);
+            }
             if (j == W - 1) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) sU[v * NL] = u[v];
@@ -943,7 +1076,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
 #pragma unroll
                         for (int k = 1; k < 6; ++k) amx = larger(amx, larger(sL[k * NL], sL[6 * CL + k * NL]));
 #pragma unroll
-                        for (int k = 0; k < 5; ++k) { dF[k] = sD[r * CD + k * NL]; dq[k] = sD[(7 + r) * CD + k * NL]; }
+                        for (int k = 0; k < 5; ++k) diff_at(r, k, dF[k], dq[k]);
                         const double lin = (double)linear_flux(dF, dq, amx);
                         const double rho = fv.rho, v2 = 2.0 * fv.hvv, b2 = fv.bbn2 * fv.rho;
                         const double pg = 0.5 * ((double)sC[CL + 2 * NL] + (double)sC[CL + 3 * NL]);
@@ -967,7 +1100,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
                     for (int r = 0; r < 7; ++r) {
                         R dF[5], dq[5];
 #pragma unroll
-                        for (int k = 0; k < 5; ++k) { dF[k] = sD[r * CD + k * NL]; dq[k] = sD[(7 + r) * CD + k * NL]; }
+                        for (int k = 0; k < 5; ++k) diff_at(r, k, dF[k], dq[k]);
                         const double lin = (double)linear_flux(dF, dq, amx) + sF[r * CP];
                         fl[r] = full ? fl[r] : lin;
                     }
@@ -1066,7 +1199,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
         {
             MoveBack<double, 12, CP, M::HP * NL> pf;   // P and F rows are adjacent
             MoveBack<double, 3, CB, M::HB * NL> vb;
-            MoveBack<R, 14, CD, M::HD * NL> d;
+            MoveBack<DT, Diff<R>::rows, CD, M::HD * NL> d;
             MoveBack<R, 7, CL, M::HL * NL> e;
             pf.load(sP - lane, lane); vb.load(sB - lane, lane); d.load(sD - lane, lane); e.load(sL - lane, lane);
             if constexpr (MODE != 0) {
