@@ -5,6 +5,7 @@
 // member of an ensemble computes exactly what the same run computes alone.
 #pragma once
 
+#include "fp_ops.cuh"
 #include "how_internal.cuh"
 
 namespace how {
@@ -168,17 +169,25 @@ __device__ __forceinline__ double warp_max(double v) {
 __device__ __forceinline__ bool op_tstep_cell(const Grid& g, const double* __restrict__ q, double gam,
                                               double rhomin, double pgmin, long long t, double& mx, double& my,
                                               double& mz) {
-    const int i = 3 + (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = 3 + (int)(r % g.ny);
-    const int k = 3 + (int)(r / g.ny);
+    int i, j, k;
+    if (t < (1ll << 32)) {   // (a 64-bit division costs as much as the cell's arithmetic)
+        const unsigned u = (unsigned)t, r = u / (unsigned)g.nx, p = r / (unsigned)g.ny;
+        i = 3 + (int)(u - r * (unsigned)g.nx);
+        j = 3 + (int)(r - p * (unsigned)g.ny);
+        k = 3 + (int)p;
+    } else {
+        const long long r = t / g.nx;
+        i = 3 + (int)(t % g.nx);
+        j = 3 + (int)(r % g.ny);
+        k = 3 + (int)(r / g.ny);
+    }
     const long long c = g.idx(i, j, k);
     const double DD = q[c], Mx = q[g.fs + c], My = q[2 * g.fs + c], Mz = q[3 * g.fs + c];
     const double Bx = q[4 * g.fs + c], By = q[5 * g.fs + c], Bz = q[6 * g.fs + c];
     const double EE = q[7 * g.fs + c];
     const double rho = fmax(DD, rhomin);
     // the seven quotients by rho, each correctly rounded, from one division
-    const double ir = 1.0 / rho;
+    const double ir = recip(rho);
     const double vx = div_const(Mx, rho, ir), vy = div_const(My, rho, ir), vz = div_const(Mz, rho, ir);
     const double vv2 = vx * vx + vy * vy + vz * vz;
     const double BB2 = Bx * Bx + By * By + Bz * Bz;
@@ -188,12 +197,12 @@ __device__ __forceinline__ bool op_tstep_cell(const Grid& g, const double* __res
     const double bnx2 = div_const(Bx * Bx, rho, ir), bny2 = div_const(By * By, rho, ir),
                  bnz2 = div_const(Bz * Bz, rho, ir);
     const double s = (bbn2 + cs2) * (bbn2 + cs2);
-    const double rootx = sqrt(fmax(0.0, s - 4.0 * bnx2 * cs2));
-    const double rooty = sqrt(fmax(0.0, s - 4.0 * bny2 * cs2));
-    const double rootz = sqrt(fmax(0.0, s - 4.0 * bnz2 * cs2));
-    const double lfx = sqrt(fmax(0.0, 0.5 * (bbn2 + cs2 + rootx)));
-    const double lfy = sqrt(fmax(0.0, 0.5 * (bbn2 + cs2 + rooty)));
-    const double lfz = sqrt(fmax(0.0, 0.5 * (bbn2 + cs2 + rootz)));
+    const double rootx = root(s - 4.0 * bnx2 * cs2);
+    const double rooty = root(s - 4.0 * bny2 * cs2);
+    const double rootz = root(s - 4.0 * bnz2 * cs2);
+    const double lfx = root(0.5 * (bbn2 + cs2 + rootx));
+    const double lfy = root(0.5 * (bbn2 + cs2 + rooty));
+    const double lfz = root(0.5 * (bbn2 + cs2 + rootz));
     mx = fmax(mx, fabs(vx) + lfx);
     my = fmax(my, fabs(vy) + lfy);
     mz = fmax(mz, fabs(vz) + lfz);
@@ -268,7 +277,7 @@ __device__ __forceinline__ void op_prot_cell(const Grid& g, double* __restrict__
     const double Bx = q[4 * g.fs + c], By = q[5 * g.fs + c], Bz = q[6 * g.fs + c];
     double E = q[7 * g.fs + c];
     rho = fmax(rho, rhomin);
-    const double irho = 1.0 / rho, igm1 = 1.0 / (gam - 1.0);
+    const double irho = recip(rho), igm1 = recip(gam - 1.0);
     const double vx = div_const(Mx, rho, irho), vy = div_const(My, rho, irho), vz = div_const(Mz, rho, irho);
     const double vv2 = vx * vx + vy * vy + vz * vz;
     const double BB2 = Bx * Bx + By * By + Bz * Bz;
@@ -459,7 +468,7 @@ __device__ __forceinline__ void op_interp_prot_cell(const Grid& g, const double*
     if (!prot_too) return;
     rho = fmax(rho, rhomin);
     // the four quotients of prot, each correctly rounded, from two divisions
-    const double irho = 1.0 / rho, igm1 = 1.0 / (gam - 1.0);
+    const double irho = recip(rho), igm1 = recip(gam - 1.0);
     const double vx = div_const(Mx, rho, irho), vy = div_const(My, rho, irho), vz = div_const(Mz, rho, irho);
     const double vv2 = vx * vx + vy * vy + vz * vz;
     const double BB2 = Bx * Bx + By * By + Bz * Bz;
