@@ -354,10 +354,15 @@ __device__ __forceinline__ void op_emf_cell(const Grid& g, const CTFields& f, in
                                             int i, int j, int k) {
     const long long c = g.idx(i, j, k);
     const long long sj = g.pitch, sk = (long long)g.pitch * g.P1;
+    // (every load before the first quotient, whose range check is a branch)
+    double x[5] = {}, y[5] = {}, z[5] = {};
+    if (use_Ox) { x[0] = f.Ox2[c]; x[1] = f.Ox2[c - 1]; x[2] = f.Ox2[c + 1]; x[3] = f.Ox2[c - sj]; x[4] = f.Ox2[c + sj]; }
+    if (use_Oy) { y[0] = f.Oy2[c]; y[1] = f.Oy2[c - sj]; y[2] = f.Oy2[c + sj]; y[3] = f.Oy2[c - sk]; y[4] = f.Oy2[c + sk]; }
+    if (use_Oz) { z[0] = f.Oz2[c]; z[1] = f.Oz2[c - 1]; z[2] = f.Oz2[c + 1]; z[3] = f.Oz2[c - sk]; z[4] = f.Oz2[c + sk]; }
     double ox = 0.0, oy = 0.0, oz = 0.0;
-    if (use_Ox) ox = ct_smooth(f.Ox2[c], f.Ox2[c - 1], f.Ox2[c + 1], f.Ox2[c - sj], f.Ox2[c + sj]);
-    if (use_Oy) oy = ct_smooth(f.Oy2[c], f.Oy2[c - sj], f.Oy2[c + sj], f.Oy2[c - sk], f.Oy2[c + sk]);
-    if (use_Oz) oz = ct_smooth(f.Oz2[c], f.Oz2[c - 1], f.Oz2[c + 1], f.Oz2[c - sk], f.Oz2[c + sk]);
+    if (use_Ox) ox = ct_smooth(x[0], x[1], x[2], x[3], x[4]);
+    if (use_Oy) oy = ct_smooth(y[0], y[1], y[2], y[3], y[4]);
+    if (use_Oz) oz = ct_smooth(z[0], z[1], z[2], z[3], z[4]);
     if (use_Ox) f.Ox[c] = ox;
     if (use_Oy) f.Oy[c] = oy;
     if (use_Oz) f.Oz[c] = oz;
