@@ -1,7 +1,7 @@
 // ensemble.cu -- batched ensembles of independent runs (members) of uneven
 // sizes.  Each kernel of an SSPRK(5,4) step is launched once for all members:
-// the sweeps as one persistent launch per direction over every member's
-// tiles (ensemble_sweep.cu), the memory-bound kernels with blocks assigned to
+// the sweeps as one launch per direction over every member's work items
+// (ensemble_sweep.cu), the memory-bound kernels with blocks assigned to
 // members by prefix sums.  The step -- CFL reduction, dt with each member's
 // own output-time clamp, five stages, time advance -- runs entirely on the
 // device, so one CUDA graph of one step is replayed until every member has
@@ -404,7 +404,7 @@ int check_status(how_ensemble* e) {
 // fastest shape.  A direction's time is its sweeps of stages 2-5, scaled by
 // 5/4: the stage-1 launch of a shape is that kernel's first, and can carry
 // its one-time module load.  The steps advance the members like any other
-// step (the tile shape does not change the arithmetic).
+// step (the shape does not change the arithmetic).
 int autotune(how_ensemble* e, long* steps_done) {
     cudaEvent_t ev[30];
     for (auto& x : ev) HOW_CUDA_CHECK(cudaEventCreate(&x));

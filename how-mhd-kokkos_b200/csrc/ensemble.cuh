@@ -7,9 +7,9 @@
 
 namespace how {
 
-constexpr int kEnsShapes = 3;   // tile-shape candidates per sweep direction
+constexpr int kEnsShapes = 3;   // work-item shapes per sweep direction
 
-// shapes, tiles and launches of the batched sweep (ensemble_sweep.cu)
+// shapes, work items and launches of the batched sweep (ensemble_sweep.cu)
 void ens_shape(int dir, int s, int* nl, int* t);
 long long ens_tiles(const Grid& g, int dir, int s);
 int ens_encode_maps(const Ctx& c, int dir, int s, CUtensorMap* tm_in, CUtensorMap* tm_out);

@@ -93,7 +93,7 @@ enum : unsigned int { HOW_STATUS_NONFINITE_DT = 1u, HOW_STATUS_TMA_TIMEOUT = 2u,
 
 // Arguments of one directional sweep launch.
 struct SweepArgs {
-    CUtensorMap tm_in;     // stage iw-1: the pencil tile (with halo) of all 8 variables
+    CUtensorMap tm_in;     // stage iw-1: a chunk's new cells, all 8 variables
     CUtensorMap tm_out;    // the update's read operand: q(iw) (accumulate) or the RK base
     Grid g;
     const double* qprev;   // stage iw-1, field 0 (vars at + v * fs)
@@ -128,12 +128,12 @@ struct SweepArgs {
     // batched ensembles (ENS kernels): member m's arguments for this launch
     // are ens_tab[m * ens_stride + ens_off + ens_par[m]]
     const SweepArgs* ens_tab;
-    const long long* ens_tile_start;   // [ens_n + 1]: prefix of the members' tile counts
+    const long long* ens_tile_start;   // [ens_n + 1]: prefix of the members' work items
     const int* ens_par;                // per member: stage-0 / stage-5 buffer parity
     const int* ens_active;             // per member: 1 while it is stepping
     int ens_n, ens_stride, ens_off;
-    // failure-detection tests: nonzero makes the compute threads' tile waits
-    // give up at once (the issuer's drain of copies in flight keeps its
+    // failure-detection tests: nonzero makes the tile waits
+    // give up at once (the drain of copies in flight keeps its
     // full limit), so the launch ends early with HOW_STATUS_TMA_TIMEOUT
     int wait_expire;
 };
@@ -164,7 +164,7 @@ struct Ctx {
     size_t mem_bytes = 0;
     double* q[6] = {};              // stage s, field 0; var v at + v * fs
     double* qbuf[6] = {};           // the six physical stage buffers (q[] is a permutation)
-    CUtensorMap tm_in[6][3];        // per physical buffer and sweep direction: input tile
+    CUtensorMap tm_in[6][3];        // per physical buffer and sweep direction: raw tile
     CUtensorMap tm_out[6][3];       // per physical buffer and sweep direction: update tile
     double* b[6] = {};              // face B stage s: comps at + c * fs
     double* ct[12] = {};            // fsy fsz gsx gsz hsx hsy Ox2 Oy2 Oz2 Ox Oy Oz

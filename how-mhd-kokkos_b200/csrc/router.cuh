@@ -1,11 +1,11 @@
-// router.cuh -- the learned WENO router's device pieces, shared by the sweep
-// kernel (inference inside a tile) and router.cu (training, batched
-// inference, gradient checks).
+// router.cuh -- the learned WENO router's device pieces, shared by the routing
+// pass (route_prepass.cu), the sweep kernel (guard, label collection) and
+// router.cu (training, batched inference, gradient checks).
 //
 // Network: 6 features -> 32 -> 32 (GELU, tanh form) -> 1 logit.  Inference
 // runs on the tensor cores with mma.sync m16n8k16 BF16 x BF16 -> FP32 and the
-// hardware tanh (the per-tile batch is at most a few dozen interfaces, far
-// below a tcgen05 128-row tile); training is FP32 (router.cu).
+// hardware tanh (a warp's batch is 32 interfaces, far below a tcgen05 128-row
+// tile); training is FP32 (router.cu).
 //
 // Features of the interface between cells c+2 and c+3 over its 6-cell
 // stencil c..c+5 (all dimensionless, log10 with a 1e-6 floor):

@@ -405,7 +405,7 @@ class Domain:
         _check(_lib.how_output_wait(self._h))
 
     def sweep_phase_profile(self, direction: int, dt: float):
-        """Mean cycles per block of each sweep phase (instrumentation)."""
+        """Mean cycles of each phase of a warp's chunk in one sweep (instrumentation)."""
         out = np.zeros(12)
         _check(_lib.how_sweep_phase_profile(self._h, direction, dt, _dptr(out), 12))
         return out

@@ -216,12 +216,10 @@ int how_get_kernel_timing(how_ctx* ctx, double* total_ms, long* launches);
  * waits, with its full limit, for every copy it has in flight before the
  * block exits.  0 restores the normal waits; the context stays usable. */
 int how_set_wait_limit(how_ctx* ctx, int expire_at_once);
-/* Mean cycles per thread block of each phase of one stage-1 sweep (the
- * how_sweep semantics) -- instrumentation, no reference counterpart.
- * out[0..10] = phases (load, primitives, cell differences, routing features,
- * routing network, routing decision, eigen-system scalars, eigenvector rows,
- * projection+WENO, back-projection+CT, update); out[11] = tiles.  A phase a
- * launch does not have adds nothing. */
+/* Mean cycles of each phase of a warp's chunk (32 cells) in one stage-1 sweep
+ * (the how_sweep semantics) -- instrumentation, no reference counterpart.
+ * out[0..10] = phases: 0 load, 1 cell values, 8 interface fluxes, 9 CT terms,
+ * 10 update, the others 0; out[11] = chunks. */
 int how_sweep_phase_profile(how_ctx* ctx, int dir, double dt, double* out, int nout);
 /* ------------------------------------------------------ batched ensembles */
 /* No counterpart in the reference (which runs one domain per job).  Many
@@ -241,7 +239,7 @@ int how_ensemble_size(const how_ensemble* e);
 how_ctx* how_ensemble_member(how_ensemble* e, int m);
 /* init_problem of every member; member times back to 0 */
 int how_ensemble_init(how_ensemble* e);
-/* Sweep tile shapes per direction (index into the candidate list of
+/* Sweep work-item shapes per direction (index into the candidate list of
  * how_ensemble_shape_info).  Without this call the first how_ensemble_run
  * autotunes: one real step per candidate, then the fastest per direction. */
 int how_ensemble_set_shapes(how_ensemble* e, int sx, int sy, int sz);
