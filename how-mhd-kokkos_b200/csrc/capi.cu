@@ -258,6 +258,7 @@ int how_create(const how_params* p, how_ctx** out) {
     c->precision = pp.precision;
     c->g = make_grid(pp.nx, pp.ny, pp.nz);
     cudaGetDevice(&c->dev);
+    cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->dev);
     const Grid& g = c->g;
     const int nfields = 6 * 8 + 6 * 3 + 12 + 8;
     c->mem_bytes = (size_t)nfields * g.fs * sizeof(double);

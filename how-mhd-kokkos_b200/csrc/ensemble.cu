@@ -219,6 +219,7 @@ struct how_ensemble {
     cudaGraphExec_t exec = nullptr;
     double sweep_ms[3][kEnsShapes] = {};
     long graph_launches = 0;
+    SmemLimits smem;
 };
 
 namespace {
@@ -337,7 +338,7 @@ void enqueue_step(how_ensemble* e, cudaEvent_t* ev) {
             a0.ens_off = (iw * 3 + d) * 2;
             a0.status = e->d_status;
             if (ev) cudaEventRecord(ev[(d * 5 + iw - 1) * 2], e->stream);
-            ens_launch_sweep(d, e->shape[d], a0, e->stream, e->dev);
+            ens_launch_sweep(d, e->shape[d], a0, e->stream, e->members[0]->sm_count, e->smem);
             if (ev) cudaEventRecord(ev[(d * 5 + iw - 1) * 2 + 1], e->stream);
         }
         // fluxct (CT members) or face-B base (1-D members), then prot and the ghost fill
@@ -440,10 +441,17 @@ int autotune(how_ensemble* e, long* steps_done) {
 
 int capture(how_ensemble* e) {
     cudaGraph_t g = nullptr;
+    const bool clean = cudaPeekAtLastError() == cudaSuccess;
     HOW_CUDA_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
     enqueue_step(e, nullptr);
-    HOW_CUDA_CHECK(cudaStreamEndCapture(e->stream, &g));
-    cudaError_t err = cudaGraphInstantiate(&e->exec, g, 0);
+    cudaError_t err = cudaStreamEndCapture(e->stream, &g);
+    // (a launch that was refused is not in the graph)
+    if (err == cudaSuccess && clean) err = cudaGetLastError();
+    if (err != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return cuda_fail(err, "capture of the ensemble's step");
+    }
+    err = cudaGraphInstantiate(&e->exec, g, 0);
     cudaGraphDestroy(g);
     if (err != cudaSuccess) { e->exec = nullptr; return cuda_fail(err, "cudaGraphInstantiate"); }
     return HOW_OK;

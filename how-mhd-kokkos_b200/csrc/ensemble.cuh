@@ -13,7 +13,7 @@ constexpr int kEnsShapes = 3;   // work-item shapes per sweep direction
 void ens_shape(int dir, int s, int* nl, int* t);
 long long ens_tiles(const Grid& g, int dir, int s);
 int ens_encode_maps(const Ctx& c, int dir, int s, CUtensorMap* tm_in, CUtensorMap* tm_out);
-void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int dev);
+void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int nsm, SmemLimits& smem);
 
 // Per-member description read by the batched kernels.  Stage s of q lives in
 // qbuf[s], except that stages 0 and 5 trade buffers when par (the member's

@@ -20,18 +20,13 @@ constexpr ShapeDef kShapes[3][kEnsShapes] = {
     {{4, 2}, {4, 8}, {2, 2}},
     {{4, 2}, {4, 8}, {4, 4}},
 };
-constexpr int kWarps = 12, kBlocks = 1;   // warps per block, blocks per SM: as the single-domain FP64 sweep
+constexpr int kWarps = 12, kBlocks = 1;   // warps per block, blocks per SM: as the single-domain FP64 sweep (nsm blocks)
 
 template <int DIR, int NL>
-void launch_ens(SweepArgs a0, int chunks, cudaStream_t st, int dev) {
+void launch_ens(SweepArgs a0, int chunks, cudaStream_t st, int nsm, SmemLimits& smem) {
     constexpr int bytes = kWarps * WarpMem<DIR, NL, double, 0>::bytes + 128;
     const auto kern = k_sweep<DIR, NL, kWarps, double, kBlocks, 0, true>;
-    static const int nsm = [&] {   // one block per SM
-        int n = 148;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n;
-    }();
+    smem.raise((const void*)kern, bytes);
     a0.seg_chunks = chunks;
     kern<<<nsm, 32 * kWarps, bytes, st>>>(a0);
 }
@@ -71,16 +66,16 @@ int ens_encode_maps(const Ctx& c, int dir, int s, CUtensorMap* tm_in, CUtensorMa
     return 0;
 }
 
-void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int dev) {
+void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int nsm, SmemLimits& smem) {
     const ShapeDef& d = kShapes[dir][s];
     if (dir == 0) {
-        if (d.nl == 1) launch_ens<0, 1>(a0, d.chunks, st, dev);
-        else launch_ens<0, 4>(a0, d.chunks, st, dev);
+        if (d.nl == 1) launch_ens<0, 1>(a0, d.chunks, st, nsm, smem);
+        else launch_ens<0, 4>(a0, d.chunks, st, nsm, smem);
     } else if (dir == 1) {
-        if (d.nl == 2) launch_ens<1, 2>(a0, d.chunks, st, dev);
-        else launch_ens<1, 4>(a0, d.chunks, st, dev);
+        if (d.nl == 2) launch_ens<1, 2>(a0, d.chunks, st, nsm, smem);
+        else launch_ens<1, 4>(a0, d.chunks, st, nsm, smem);
     } else {
-        launch_ens<2, 4>(a0, d.chunks, st, dev);
+        launch_ens<2, 4>(a0, d.chunks, st, nsm, smem);
     }
 }
 

@@ -155,10 +155,25 @@ struct StepGraph {
     int seen = 0;   // steps taken launch by launch since the last change
 };
 
+// A kernel's dynamic shared-memory limit belongs to a device, and goes with a
+// device reset: the owner of launches past the default 48 KB (a context, an
+// ensemble) raises it once for each kernel it launches.  A refusal is left as
+// the runtime's last error, as the launch's own failure is, and asked for again.
+struct SmemLimits {
+    std::vector<const void*> raised;
+    void raise(const void* kernel, int bytes) {
+        for (const void* k : raised) if (k == kernel) return;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+            raised.push_back(kernel);
+    }
+};
+
 struct Ctx {
     how_params p;
     Grid g;
     int dev = 0;
+    int sm_count = 148;             // of the device
+    SmemLimits smem;
     cudaStream_t stream = nullptr;
     double* mem = nullptr;          // one allocation for every field
     size_t mem_bytes = 0;

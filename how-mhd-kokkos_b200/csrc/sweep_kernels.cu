@@ -31,25 +31,15 @@ Plan pick_chunks(const Grid& g, int nsm, int warps) {
     return best;
 }
 
-int sm_count(const Ctx& c) {
-    static const int n = [&] {
-        int v = 148;
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, c.dev);
-        return v;
-    }();
-    return n;
-}
-
 template <int DIR, int WPB, typename R, int MODE>
 void launch_plan(Ctx& c, SweepArgs& a, const Plan& plan) {
     constexpr int bytes = WPB * WarpMem<DIR, kLines, R, MODE>::bytes + 128;
     const auto kern = k_sweep<DIR, kLines, WPB, R, 1, MODE>;
-    static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    (void)set;
+    c.smem.raise((const void*)kern, bytes);
     a.seg_chunks = plan.chunks;
     // persistent grid: one block per SM (a kernel with tensor memory)
     const long long items = Cut<DIR, kLines>(c.g, plan.chunks).items();
-    const int nsm = sm_count(c), grid = (int)(items < nsm ? items : nsm);
+    const int grid = (int)(items < c.sm_count ? items : c.sm_count);
     cudaEvent_t ev[2];
     timer_begin(c, ev);
     kern<<<grid, 32 * WPB, bytes, c.stream>>>(a);
@@ -61,7 +51,7 @@ void launch_plan(Ctx& c, SweepArgs& a, const Plan& plan) {
 // SMALL / 4 items
 template <int DIR, int WPB, int SMALL, typename R, int MODE>
 void launch_one(Ctx& c, SweepArgs& a) {
-    const Plan plan = pick_chunks<DIR>(c.g, sm_count(c), WPB / 4);
+    const Plan plan = pick_chunks<DIR>(c.g, c.sm_count, WPB / 4);
     if constexpr (SMALL > 0)
         if (plan.each <= SMALL / 4) return launch_plan<DIR, SMALL, R, MODE>(c, a, plan);
     launch_plan<DIR, WPB, R, MODE>(c, a, plan);

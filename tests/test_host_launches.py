@@ -1,0 +1,140 @@
+"""What the library's host side asks of CUDA, without a GPU: the built objects
+linked against tests/fake_cuda.cpp, which counts launches, captures and graph
+replays and refuses what the runtime refuses (a launch with more dynamic shared
+memory than the kernel's limit on that device)."""
+import ctypes
+import importlib.util
+import os
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+PKG = Path(__file__).resolve().parents[1] / "how-mhd-kokkos_b200"
+
+
+@pytest.fixture(scope="module")
+def module(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not found")
+    objs = [PKG / "_build" / (f.stem + ".o") for f in (PKG / "csrc").iterdir()
+            if f.suffix in (".cu", ".cpp") and f.name != "driver_main.cpp"]
+    if not all(o.exists() for o in objs):
+        pytest.skip("the library's objects are not built")
+    so = tmp_path_factory.mktemp("fake") / "libhowfake.so"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-o", str(so),
+                    str(Path(__file__).with_name("fake_cuda.cpp")), *map(str, objs), "-lgomp", "-ldl", "-lpthread"],
+                   check=True)
+    old = os.environ.get("HOW_MHD_LIB")
+    os.environ["HOW_MHD_LIB"] = str(so)
+    try:
+        spec = importlib.util.spec_from_file_location("how_mhd_fake", PKG / "how_mhd" / "__init__.py")
+        hm = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(hm)
+    finally:
+        if old is None:
+            del os.environ["HOW_MHD_LIB"]
+        else:
+            os.environ["HOW_MHD_LIB"] = old
+    fake = ctypes.CDLL(str(so))
+    fake.fake_launches.restype = ctypes.c_char_p
+    fake.fake_calls.restype = ctypes.c_long
+    return hm, fake
+
+
+@pytest.fixture
+def lib(module):
+    hm, fake = module
+    fake.fake_reset(2)
+    yield hm, fake
+    fake.fake_reset(1)
+
+
+def _params(hm, n, bc="periodic", **kw):
+    return hm.make_parameters(nx=n[0], ny=n[1], nz=n[2], nt=1, tend=1.0, gam=5.0 / 3.0, cour=0.4, problem="uniform",
+                              x1bc=bc, x2bc=bc, x3bc=bc, **kw)
+
+
+class Launch:
+    def __init__(self, row):
+        captured, device, grid, block, smem, self.kernel = row.split(" ", 5)
+        self.captured, self.device, self.smem = captured == "1", int(device), int(smem)
+        self.blocks = int(grid.split(",")[0])
+
+
+def _launches(fake, kernel=""):
+    """The launches since the last call, of the kernels with this name."""
+    rows = map(Launch, fake.fake_launches().decode().splitlines())
+    return [r for r in rows if kernel in r.kernel]
+
+
+@pytest.mark.parametrize("kw", [{}, {"precision": "mixed"}, {"precision": "mixed", "router": "on"}],
+                         ids=["fp64", "mixed", "routed"])
+def test_a_second_device_gets_its_own_limits(lib, kw):
+    """The sweeps' shared memory is past the default limit, which is raised per
+    device: a second domain on another device, and one after a device reset."""
+    hm, fake = lib
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        with hm.Domain(_params(hm, (40, 37, 35), **kw)) as d:
+            _launches(fake)
+            d.ssprk(1e-3)
+            rows = _launches(fake, "k_sweep")
+            assert len(rows) == 15 and all(r.device == device and r.smem > 49152 for r in rows)
+            # persistent blocks: at most as many as this device has SMs
+            assert max(r.blocks for r in rows) <= (148, 100)[device]
+    fake.cudaDeviceReset()
+    with hm.Domain(_params(hm, (40, 37, 35), **kw)) as d:
+        d.ssprk(1e-3)
+
+
+def test_a_group_over_two_devices_launches(lib):
+    hm, fake = lib
+    p = _params(hm, (20, 18, 16))
+    with hm.Group(p, 2, devices=[0, 1]) as g:
+        g.set_state(np.ones((8, 26, 24, 22)))
+        _launches(fake)
+        with pytest.raises(hm.HowError, match="non-positive dt"):   # (no device: no dt)
+            g.run(0.0, 1)
+        assert {r.device for r in _launches(fake)} == {0, 1}
+    for k in (0, 1):   # the parts' own steps
+        fake.fake_set_device(k)
+        with hm.Domain(p) as d:
+            d.ssprk(1e-3)
+
+
+def test_an_ensemble_on_a_second_device_launches(lib):
+    hm, fake = lib
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        with hm.Ensemble([_params(hm, (40, 1, 1)), _params(hm, (24, 20, 1))]) as e:
+            e.init()
+            e.set_shapes(0, 1, 0)
+            _launches(fake)
+            e.run(1)
+            rows = _launches(fake, "k_sweep")   # x sweeps, and y sweeps of the 2-D member
+            assert len(rows) == 10 and all(r.captured and r.device == device for r in rows)
+
+
+def test_an_ensemble_does_not_run_without_its_sweeps(lib):
+    hm, fake = lib
+    with hm.Ensemble([_params(hm, (40, 1, 1)), _params(hm, (24, 20, 1))]) as e:
+        e.init()
+        e.set_shapes(0, 0, 0)
+        fake.fake_fail(b"cudaFuncSetAttribute", 999)
+        with pytest.raises(hm.HowError):
+            e.run(1)
+        fake.fake_fail(b"cudaFuncSetAttribute", 0)
+        e.run(1)
+
+
+def test_a_refused_limit_is_an_error_and_is_asked_for_again(lib):
+    hm, fake = lib
+    with hm.Domain(_params(hm, (40, 37, 35))) as d:
+        fake.fake_fail(b"cudaFuncSetAttribute", 999)
+        with pytest.raises(hm.HowError):
+            d.ssprk(1e-3)
+        fake.fake_fail(b"cudaFuncSetAttribute", 0)
+        d.ssprk(1e-3)
