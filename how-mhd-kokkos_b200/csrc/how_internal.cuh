@@ -145,14 +145,14 @@ struct RouterLayout {
                          ob3 = ow3 + H, total = ob3 + 1;
 };
 
-// The launches of one SSPRK step as a CUDA graph, for the buffers and settings
-// it was captured with (capi.cu).
+// The launches of one SSPRK step as a CUDA graph, for the buffers it was
+// captured with (capi.cu).
 struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     const double *q0 = nullptr, *b0 = nullptr;
-    int settings = 0;
     long launches = 0;
-    int seen = 0;   // steps taken launch by launch since the last change
+    int seen = 0;           // steps taken launch by launch
+    bool refused = false;   // launch by launch for good
 };
 
 // A kernel's dynamic shared-memory limit belongs to a device, and goes with a
@@ -215,7 +215,7 @@ struct Ctx {
     // reach every buffer) fill axis by axis, as the standalone entry points do.
     bool one_pass_fill = false;
     int axis_fill_steps = 0;
-    StepGraph step_graph[2];              // one for each role of the stage-0 / stage-5 buffers
+    StepGraph step_graph[2][2];           // [precision][role of the stage-0 / stage-5 buffers]
     int wait_expire = 0;                  // failure-detection test hook (SweepArgs::wait_expire)
     // part of a domain decomposed into z slabs (how_group_*): the global z
     // index of local plane 3 minus 3, and which z ghost layers this context

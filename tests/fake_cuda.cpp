@@ -89,7 +89,7 @@ int __cudaPopCallConfiguration(Dim* g, Dim* b, size_t* smem, void** stream) {
     return 0;
 }
 int cudaLaunchKernel(const void* f, Dim g, Dim b, void**, size_t smem, void*) {
-    const int e = enter("cudaLaunchKernel");
+    const int e = enter(capturing ? "captured launch" : "cudaLaunchKernel");
     if (e) return e;
     std::lock_guard<std::mutex> l(mu);
     const auto lim = smem_limit.find({device, f});

@@ -130,6 +130,73 @@ def test_an_ensemble_does_not_run_without_its_sweeps(lib):
         e.run(1)
 
 
+def _step(d, n):
+    for _ in range(n):
+        d.ssprk(1e-3)
+
+
+@pytest.mark.parametrize("n", [(48, 1, 1), (24, 20, 1), (12, 10, 9)], ids=["1d", "2d", "3d"])
+def test_steps_become_a_graph_per_buffer_role(lib, n):
+    hm, fake = lib
+    with hm.Domain(_params(hm, n)) as d:
+        _step(d, 60)
+        assert fake.fake_calls(b"cudaGraphInstantiate") == 2
+        assert fake.fake_calls(b"cudaGraphLaunch") == 60 - 16
+
+
+def test_a_written_state_keeps_the_graphs(lib):
+    """A periodic axis of one cell: the two steps after a state was written fill
+    axis by axis, beside the graphs."""
+    hm, fake = lib
+    with hm.Domain(_params(hm, (24, 20, 1))) as d:
+        q = np.ones((8, 30, 26, 7))
+        _step(d, 20)
+        for _ in range(5):
+            d.set_state(q)
+            _step(d, 20)
+        assert fake.fake_calls(b"cudaGraphInstantiate") == 2 and fake.fake_calls(b"cudaGraphExecDestroy") == 0
+        assert fake.fake_calls(b"cudaGraphLaunch") == 4 + 5 * 18
+
+
+def test_a_change_of_precision_keeps_the_graphs(lib):
+    hm, fake = lib
+    with hm.Domain(_params(hm, (12, 10, 9))) as d:
+        for _ in range(4):
+            for precision in ("mixed", "fp64"):
+                d.set_precision(precision)
+                _step(d, 20)
+        assert fake.fake_calls(b"cudaGraphInstantiate") == 4
+        assert fake.fake_calls(b"cudaGraphLaunch") == 2 * (4 + 3 * 20)
+
+
+@pytest.mark.parametrize("call", ["cudaStreamBeginCapture", "cudaStreamEndCapture", "cudaGraphInstantiate",
+                                  "cudaGraphLaunch"])
+def test_a_step_that_cannot_be_a_graph_is_launched(lib, call):
+    hm, fake = lib
+    with hm.Domain(_params(hm, (12, 10, 9))) as d:
+        _step(d, 16)
+        _launches(fake)
+        fake.fake_fail(call.encode(), 901)
+        _step(d, 30)
+        rows = [r for r in _launches(fake, "k_sweep") if not r.captured]
+        assert len(rows) == 30 * 15
+        assert fake.fake_calls(call.encode()) == 2   # once per buffer role, then no more
+
+
+def test_a_launch_refused_in_a_capture_is_not_left_out(lib):
+    hm, fake = lib
+    with hm.Domain(_params(hm, (12, 10, 9))) as d:
+        _step(d, 16)
+        _launches(fake)
+        fake.fake_fail(b"captured launch", 1)
+        _step(d, 4)
+        assert len(_launches(fake, "k_sweep")) == 4 * 15
+        assert fake.fake_calls(b"cudaGraphLaunch") == 0
+        fake.fake_fail(b"cudaLaunchKernel", 1)   # a refused launch of the step itself is its error
+        with pytest.raises(hm.HowError):
+            d.ssprk(1e-3)
+
+
 def test_a_refused_limit_is_an_error_and_is_asked_for_again(lib):
     hm, fake = lib
     with hm.Domain(_params(hm, (40, 37, 35))) as d:
