@@ -14,7 +14,9 @@ constexpr int kLines = 4;   // lines per warp: 32-byte rows in y and z
 // busiest quarter of an SM, which holds `warps` warps at once.  A chunk takes
 // about 1 + w units of time with w warps beside one another (4.3k cycles alone
 // and 14k among three, FP64), and a segment's first five cells, which have no
-// interface yet, a quarter of a chunk.
+// interface yet, a quarter of a chunk.  Once no quarter gets a second item,
+// longer ones only take longer: the search ends there (8 us at 5e6 cells of one
+// line, where trying every length takes 5 ms).
 struct Plan { int chunks; long long each; };   // each: items per quarter of an SM
 template <int DIR>
 Plan pick_chunks(const Grid& g, int nsm, int warps) {
@@ -27,6 +29,7 @@ Plan pick_chunks(const Grid& g, int nsm, int warps) {
         const long long each = (CUT(g, s).items() + 4 * nsm - 1) / (4 * nsm), rest = each % warps;
         const double t = (double)(each / warps * (1 + warps) + (rest ? 1 + rest : 0)) * (s + 0.25);
         if (s == 1 || t < best_t) { best = Plan{s, each}; best_t = t; }
+        if (each <= 1) break;
     }
     return best;
 }

@@ -7,6 +7,7 @@ import importlib.util
 import os
 import shutil
 import subprocess
+import time
 from pathlib import Path
 
 import numpy as np
@@ -195,6 +196,19 @@ def test_a_launch_refused_in_a_capture_is_not_left_out(lib):
         fake.fake_fail(b"cudaLaunchKernel", 1)   # a refused launch of the step itself is its error
         with pytest.raises(hm.HowError):
             d.ssprk(1e-3)
+
+
+def test_cutting_a_long_line_takes_no_time(lib):
+    """How a sweep is cut is worked out at its launch: at 2e6 cells under 1 ms
+    of a step (trying every length took 11 ms here, the launches take 0.05)."""
+    hm, fake = lib
+    with hm.Domain(_params(hm, (2000000, 1, 1), router="on")) as d:
+        took = []
+        for _ in range(5):
+            t = time.perf_counter()
+            d.ssprk(1e-3)
+            took.append(time.perf_counter() - t)
+    assert min(took) < 1e-3
 
 
 def test_a_refused_limit_is_an_error_and_is_asked_for_again(lib):
