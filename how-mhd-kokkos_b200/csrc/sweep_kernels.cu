@@ -8,19 +8,32 @@ namespace how {
 
 namespace {
 
-constexpr int kLines = 4;   // lines per warp: 32-byte rows in y and z
+// Lines per warp: four, whose rows are 32 bytes in y and z.  An x sweep takes one
+// line per warp, in chunks of 32 cells, where that makes 18% less chunks of
+// the domain, that is where lanes would be left without a line (1, 2, 3, 5, 6 or
+// 9 lines a plane, not too short).  FP64 x sweep with four lines and with one:
+// 1e5 cells of one line 75 and 26 us, 1024 x 1 x 1024 623 and 168, 1024 x 3 x 400
+// 279 and 201, 1024 x 5 x 200 280 and 164; 96^3, where no lane is idle, 186 and 191.
+constexpr int kLines = 4;
+template <int NL> double line_chunks(const Grid& g) {   // of a plane, with a quarter for each line's start
+    using CUT = Cut<0, NL>;
+    return CUT(g, 1).groups * ((g.nx - CUT::f0) / CUT::W + 1.25);
+}
+int sweep_lines(const Grid& g, int dir) {
+    return dir == 0 && line_chunks<1>(g) <= 0.82 * line_chunks<kLines>(g) ? 1 : kLines;
+}
 
 // Length of the work items, in chunks: the one with the least time on the
 // busiest quarter of an SM, which holds `warps` warps at once.  A chunk takes
 // about 1 + w units of time with w warps beside one another (4.3k cycles alone
 // and 14k among three, FP64), and a segment's first five cells, which have no
 // interface yet, a quarter of a chunk.  Once no quarter gets a second item,
-// longer ones only take longer: the search ends there (8 us at 5e6 cells of one
-// line, where trying every length takes 5 ms).
+// longer ones only take longer: the search ends there (at 2e6 cells in one line
+// trying every length takes 2 ms).
 struct Plan { int chunks; long long each; };   // each: items per quarter of an SM
-template <int DIR>
+template <int DIR, int NL>
 Plan pick_chunks(const Grid& g, int nsm, int warps) {
-    using CUT = Cut<DIR, kLines>;
+    using CUT = Cut<DIR, NL>;
     const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
     const int most = (n - CUT::f0) / CUT::W + 1;
     Plan best{1, 0};
@@ -34,14 +47,14 @@ Plan pick_chunks(const Grid& g, int nsm, int warps) {
     return best;
 }
 
-template <int DIR, int WPB, typename R, int MODE>
+template <int DIR, int NL, int WPB, typename R, int MODE>
 void launch_plan(Ctx& c, SweepArgs& a, const Plan& plan) {
-    constexpr int bytes = WPB * WarpMem<DIR, kLines, R, MODE>::bytes + 128;
-    const auto kern = k_sweep<DIR, kLines, WPB, R, 1, MODE>;
+    constexpr int bytes = WPB * WarpMem<DIR, NL, R, MODE>::bytes + 128;
+    const auto kern = k_sweep<DIR, NL, WPB, R, 1, MODE>;
     c.smem.raise((const void*)kern, bytes);
     a.seg_chunks = plan.chunks;
     // persistent grid: one block per SM (a kernel with tensor memory)
-    const long long items = Cut<DIR, kLines>(c.g, plan.chunks).items();
+    const long long items = Cut<DIR, NL>(c.g, plan.chunks).items();
     const int grid = (int)(items < c.sm_count ? items : c.sm_count);
     cudaEvent_t ev[2];
     timer_begin(c, ev);
@@ -52,22 +65,36 @@ void launch_plan(Ctx& c, SweepArgs& a, const Plan& plan) {
 
 // WPB warps per SM; SMALL (0: none) where no quarter of an SM gets more than
 // SMALL / 4 items
+template <int DIR, int NL, int WPB, int SMALL, typename R, int MODE>
+void launch_lines(Ctx& c, SweepArgs& a) {
+    const Plan plan = pick_chunks<DIR, NL>(c.g, c.sm_count, WPB / 4);
+    if constexpr (SMALL > 0)
+        if (plan.each <= SMALL / 4) return launch_plan<DIR, NL, SMALL, R, MODE>(c, a, plan);
+    launch_plan<DIR, NL, WPB, R, MODE>(c, a, plan);
+}
+
 template <int DIR, int WPB, int SMALL, typename R, int MODE>
 void launch_one(Ctx& c, SweepArgs& a) {
-    const Plan plan = pick_chunks<DIR>(c.g, c.sm_count, WPB / 4);
-    if constexpr (SMALL > 0)
-        if (plan.each <= SMALL / 4) return launch_plan<DIR, SMALL, R, MODE>(c, a, plan);
-    launch_plan<DIR, WPB, R, MODE>(c, a, plan);
+    if constexpr (DIR == 0)
+        if (sweep_lines(c.g, DIR) == 1) return launch_lines<DIR, 1, WPB, SMALL, R, MODE>(c, a);
+    launch_lines<DIR, kLines, WPB, SMALL, R, MODE>(c, a);
+}
+
+template <int DIR, int NL>
+int make_maps_lines(Ctx& c) {
+    using M = WarpMem<DIR, NL, double, 0>;   // the TMA boxes do not depend on R or MODE
+    for (int b = 0; b < 6; ++b) {
+        int rc = encode_sweep_maps(c.g, DIR, NL, M::W, M::TO, c.qbuf[b], &c.tm_in[b][DIR], &c.tm_out[b][DIR]);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 template <int DIR>
 int make_maps_dir(Ctx& c) {
-    using M = WarpMem<DIR, kLines, double, 0>;   // the TMA boxes do not depend on R or MODE
-    for (int b = 0; b < 6; ++b) {
-        int rc = encode_sweep_maps(c.g, DIR, kLines, M::W, M::TO, c.qbuf[b], &c.tm_in[b][DIR], &c.tm_out[b][DIR]);
-        if (rc) return rc;
-    }
-    return 0;
+    if constexpr (DIR == 0)
+        if (sweep_lines(c.g, DIR) == 1) return make_maps_lines<DIR, 1>(c);
+    return make_maps_lines<DIR, kLines>(c);
 }
 
 }  // namespace

@@ -198,6 +198,19 @@ def test_a_launch_refused_in_a_capture_is_not_left_out(lib):
             d.ssprk(1e-3)
 
 
+@pytest.mark.parametrize("kw", [{}, {"precision": "mixed"}, {"router": "on"}], ids=["fp64", "mixed", "routed"])
+def test_sweeps_of_few_lines_leave_no_lane_idle(lib, kw):
+    """x sweeps of one, two, three, five lines a plane: a line per warp; else four."""
+    hm, fake = lib
+    for n, lines in (((40000, 1, 1), 1), ((300, 1, 300), 1), ((300, 3, 1), 1), ((300, 5, 20), 1), ((5, 5, 300), 4),
+                     ((300, 4, 1), 4), ((300, 7, 1), 4), ((300, 300, 1), 4), ((40, 40, 40), 4)):
+        with hm.Domain(_params(hm, n, **kw)) as d:
+            _launches(fake)
+            d.ssprk(1e-3)
+            x = _launches(fake, "k_sweepILi0E")
+            assert len(x) == 5 and all("k_sweepILi0ELi%dE" % lines in r.kernel for r in x)
+
+
 def test_cutting_a_long_line_takes_no_time(lib):
     """How a sweep is cut is worked out at its launch: at 2e6 cells under 1 ms
     of a step (trying every length took 11 ms here, the launches take 0.05)."""
