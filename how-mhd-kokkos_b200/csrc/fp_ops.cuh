@@ -15,7 +15,10 @@ __device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_r
 // (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
 // 1970): the residual e of the approximation enters through the series
 // 1/(1-e) = 1 + e + e^2 and (1-e)^(-1/2) = 1 + e/2 + 3 e^2/8, whose next term
-// is below 2^-60.  recip and root end with the correction by the exact
+// is below 2^-59.  The approximations have 21 significant bits (their low words
+// are zero), so their squares are exact, and e is rounded once.  Largest errors
+// measured: near_recip 0.506 and root_inverse 0.507 units in the last place,
+// CUDA's rsqrt 0.507.  recip and root end with the correction by the exact
 // remainder (Markstein 1990), which leaves the correctly rounded result.
 // The library's sqrt() holds the FP64 pipe for 49 cycles per warp and has a
 // latency of 250 cycles (measured on one SM); root's nine operations hold it
@@ -23,7 +26,7 @@ __device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_r
 //
 // Nothing here branches or calls: selects stand in for the ends of the range.
 
-// 1 / x to about an ulp (|x| in [2^-1022, 2^1022)), and correctly rounded
+// 1 / x to 0.506 ulp (|x| in [2^-1022, 2^1022)), and correctly rounded
 __device__ __forceinline__ double near_recip(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -39,11 +42,11 @@ __device__ __forceinline__ double recip(double x) {
 }
 __device__ __forceinline__ float near_recip(float x) { return __fdividef(1.0f, x); }
 
-// 1 / sqrt(x) to about an ulp, for finite x >= 2^-1022
+// 1 / sqrt(x) to 0.507 ulp, for finite x >= 2^-1022
 __device__ __forceinline__ double root_inverse(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fm(-(x * y), y, 1.0);
+    const double e = fm(-x, y * y, 1.0);
     return fm(y * e, fm(0.375, e, 0.5), y);
 }
 __device__ __forceinline__ float root_inverse(float x) { return rsqrtf(x); }

@@ -437,7 +437,9 @@ __device__ __forceinline__ void face_values(const double* sP, const double* sB, 
     const R idf = root_inverse(df);
     const R af = wide ? root(cs2 - ls * ls) * idf : R(1), as = wide ? root(lf * lf - cs2) * idf : R(1);
     const R hvv = R(0.5) * vv2, sqr = rho * isqr;
-    const R ics2 = near_recip(cs2);
+    R ics2;
+    if constexpr (std::is_same<R, double>::value) ics2 = recip(cs2);
+    else ics2 = near_recip(cs2);
     const R sgnB = (Bx >= R(0)) ? R(1) : R(-1);
     const R btv = fm(bty, vy, btz * vz);
 
