@@ -149,23 +149,23 @@ static void run_stage(Ctx& c, int iw) {
     nvtxRangePop();
 }
 
-// The step's launches (56 in 3-D) as one graph launch, a graph for each precision
-// and buffer role.  Per step, launch by launch and as a graph: 1-D 800 cells 167
-// and 116 us, 128^2 411 and 330, 32^3 470 and 377, 64^3 1353 and 1243, 192^3
-// 22.80 and 22.66 ms.  Plain and mixed steps only (the routed step's launches
-// change with its refresh).  Steps that fill axis by axis, time or profile their
-// launches or run the wait limit's test go launch by launch and leave the graphs
-// as they are.  A capture costs what ten graph steps save, so the first eight
-// steps of each graph run launch by launch: short runs do not pay for it.  False:
-// the caller launches; where the graph's own calls are refused, from here on, and
-// their error is not the step's.
+// The step's launches (56 in 3-D) as one graph launch, a graph for each buffer
+// role.  Per step, launch by launch and as a graph: 1-D 800 cells 167 and 116 us,
+// 128^2 411 and 330, 32^3 470 and 377, 64^3 1353 and 1243, 192^3 22.80 and 22.66
+// ms.  Plain and mixed steps only (the routed step's launches change with its
+// refresh).  Steps that fill axis by axis, time or profile their launches or run
+// the wait limit's test go launch by launch and leave the graphs as they are; a
+// change of precision drops them.  A capture costs what ten graph steps save, so
+// the first eight steps with each role run launch by launch: short runs do not pay
+// for it.  False: the caller launches; where the graph's own calls are refused,
+// from here on, and their error is not the step's.
 static bool run_step_graph(Ctx& c) {
     if (c.route_mode != 0 || c.prof || timer_on(c) || !c.one_pass_fill || c.wait_expire) return false;
-    StepGraph& s = c.step_graph[c.precision == HOW_PREC_MIXED][c.q[0] == c.qbuf[0] ? 0 : 1];
-    if (s.q0 != c.q[0] || s.b0 != c.b[0]) {
+    StepGraph& s = c.step_graph[c.q[0] == c.qbuf[0] ? 0 : 1];
+    if (s.q0 != c.q[0] || s.b0 != c.b[0] || s.precision != c.precision) {
         if (s.exec) cudaGraphExecDestroy(s.exec);
         s = StepGraph{};
-        s.q0 = c.q[0]; s.b0 = c.b[0];
+        s.q0 = c.q[0]; s.b0 = c.b[0]; s.precision = c.precision;
     }
     if (s.refused || cudaPeekAtLastError() != cudaSuccess) return false;
     if (!s.exec) {
@@ -299,8 +299,7 @@ int how_destroy(how_ctx* c) {
     cudaSetDevice(c->dev);
     dump_release(*c);   // an asynchronous dump still being written finishes first
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (auto& graphs : c->step_graph)
-        for (StepGraph& s : graphs) if (s.exec) cudaGraphExecDestroy(s.exec);
+    for (StepGraph& s : c->step_graph) if (s.exec) cudaGraphExecDestroy(s.exec);
     if (c->mem) cudaFree(c->mem);
     if (c->router_w) cudaFree(c->router_w);
     if (c->route_prev) cudaFree(c->route_prev);

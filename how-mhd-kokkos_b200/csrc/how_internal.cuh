@@ -150,6 +150,7 @@ struct RouterLayout {
 struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     const double *q0 = nullptr, *b0 = nullptr;
+    int precision = 0;
     long launches = 0;
     int seen = 0;           // steps taken launch by launch
     bool refused = false;   // launch by launch for good
@@ -215,7 +216,7 @@ struct Ctx {
     // reach every buffer) fill axis by axis, as the standalone entry points do.
     bool one_pass_fill = false;
     int axis_fill_steps = 0;
-    StepGraph step_graph[2][2];           // [precision][role of the stage-0 / stage-5 buffers]
+    StepGraph step_graph[2];              // one for each role of the stage-0 / stage-5 buffers
     int wait_expire = 0;                  // failure-detection test hook (SweepArgs::wait_expire)
     // part of a domain decomposed into z slabs (how_group_*): the global z
     // index of local plane 3 minus 3, and which z ghost layers this context

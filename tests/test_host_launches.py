@@ -159,15 +159,17 @@ def test_a_written_state_keeps_the_graphs(lib):
         assert fake.fake_calls(b"cudaGraphLaunch") == 4 + 5 * 18
 
 
-def test_a_change_of_precision_keeps_the_graphs(lib):
+def test_a_change_of_precision_drops_the_graphs(lib):
     hm, fake = lib
     with hm.Domain(_params(hm, (12, 10, 9))) as d:
-        for _ in range(4):
-            for precision in ("mixed", "fp64"):
-                d.set_precision(precision)
-                _step(d, 20)
-        assert fake.fake_calls(b"cudaGraphInstantiate") == 4
-        assert fake.fake_calls(b"cudaGraphLaunch") == 2 * (4 + 3 * 20)
+        _step(d, 20)
+        d.set_precision("mixed")
+        _launches(fake)
+        _step(d, 16)
+        assert len(_launches(fake, "k_sweep")) == 16 * 15
+        _step(d, 4)
+        assert fake.fake_calls(b"cudaGraphInstantiate") == 4 and fake.fake_calls(b"cudaGraphExecDestroy") == 2
+        assert fake.fake_calls(b"cudaGraphLaunch") == 4 + 4
 
 
 @pytest.mark.parametrize("call", ["cudaStreamBeginCapture", "cudaStreamEndCapture", "cudaGraphInstantiate",
