@@ -216,6 +216,7 @@ struct how_ensemble {
     long long n_cell[CL_COUNT] = {}, n_bound[3][BK_COUNT] = {}, n_tstep = 0, n_tiles[3] = {};
     SweepArgs* d_tab = nullptr;
     int shape[3] = {-1, -1, -1};
+    int chunks[3] = {1, 1, 1};         // per work item of each direction's sweep
     cudaGraphExec_t exec = nullptr;
     double sweep_ms[3][kEnsShapes] = {};
     long graph_launches = 0;
@@ -287,8 +288,21 @@ int build_sweep_tables(how_ensemble* e) {
     if (!e->d_tab) HOW_CUDA_CHECK(cudaMalloc(&e->d_tab, tab.size() * sizeof(SweepArgs)));
     HOW_CUDA_CHECK(cudaMemcpy(e->d_tab, tab.data(), tab.size() * sizeof(SweepArgs), cudaMemcpyHostToDevice));
     for (int d = 0; d < 3; ++d) {
-        std::vector<long long> cnt(nm);
-        for (int m = 0; m < nm; ++m) cnt[m] = ens_tiles(e->members[m]->g, d, e->shape[d]);
+        // the shape's chunks, or one where so few items make a sweep as long as
+        // its longest (32 members of 200 cells, a step: 316 us with the shape's two
+        // chunks and 291 with one; one member of 200 cells 205 and 180)
+        std::vector<long long> cnt(nm), ones(nm);
+        const int chunks = ens_chunks(d, e->shape[d]), nsm = e->members[0]->sm_count;
+        long long items = 0, singles = 0;
+        int longest = 0;
+        for (int m = 0; m < nm; ++m) {
+            longest = std::max(longest, std::min(chunks, ens_line_chunks(e->members[m]->g, d, e->shape[d])));
+            items += cnt[m] = ens_tiles(e->members[m]->g, d, e->shape[d], chunks);
+            singles += ones[m] = ens_tiles(e->members[m]->g, d, e->shape[d], 1);
+        }
+        const bool short_items = sweep_time(singles, 1, nsm, 3) < 0.9 * sweep_time(items, longest, nsm, 3);
+        e->chunks[d] = short_items ? 1 : chunks;
+        if (short_items) cnt = ones;
         int rc = upload_prefix(e, e->p_tiles[d], cnt, &e->n_tiles[d]);
         if (rc) return rc;
     }
@@ -338,7 +352,7 @@ void enqueue_step(how_ensemble* e, cudaEvent_t* ev) {
             a0.ens_off = (iw * 3 + d) * 2;
             a0.status = e->d_status;
             if (ev) cudaEventRecord(ev[(d * 5 + iw - 1) * 2], e->stream);
-            ens_launch_sweep(d, e->shape[d], a0, e->stream, e->members[0]->sm_count, e->smem);
+            ens_launch_sweep(d, e->shape[d], e->chunks[d], e->n_tiles[d], a0, e->stream, e->members[0]->sm_count, e->smem);
             if (ev) cudaEventRecord(ev[(d * 5 + iw - 1) * 2 + 1], e->stream);
         }
         // fluxct (CT members) or face-B base (1-D members), then prot and the ghost fill

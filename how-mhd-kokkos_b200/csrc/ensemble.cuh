@@ -11,9 +11,12 @@ constexpr int kEnsShapes = 3;   // work-item shapes per sweep direction
 
 // shapes, work items and launches of the batched sweep (ensemble_sweep.cu)
 void ens_shape(int dir, int s, int* nl, int* t);
-long long ens_tiles(const Grid& g, int dir, int s);
+int ens_chunks(int dir, int s);                      // the shape's chunks per work item
+int ens_line_chunks(const Grid& g, int dir, int s);  // a whole line's
+long long ens_tiles(const Grid& g, int dir, int s, int chunks);
 int ens_encode_maps(const Ctx& c, int dir, int s, CUtensorMap* tm_in, CUtensorMap* tm_out);
-void ens_launch_sweep(int dir, int s, const SweepArgs& a0, cudaStream_t st, int nsm, SmemLimits& smem);
+void ens_launch_sweep(int dir, int s, int chunks, long long items, const SweepArgs& a0, cudaStream_t st, int nsm,
+                      SmemLimits& smem);
 
 // Per-member description read by the batched kernels.  Stage s of q lives in
 // qbuf[s], except that stages 0 and 5 trade buffers when par (the member's

@@ -260,6 +260,16 @@ int encode_sweep_maps(const Grid& g, int dir, int lines, int cells, int op_cells
                       CUtensorMap* out);
 void launch_copy_fields(Ctx& c, double* dst, const double* src, int nfields);
 
+// The time of a sweep cut into `items` work items of `chunks` chunks: that of
+// the busiest quarter of an SM, which holds `warps` warps at once.  A chunk
+// takes about 1 + w units of time with w warps beside one another (4.3k cycles
+// alone and 14k among three, FP64), and an item's first five cells, which have
+// no interface yet, a quarter of a chunk.
+inline double sweep_time(long long items, int chunks, int nsm, int warps) {
+    const long long each = (items + 4 * nsm - 1) / (4 * nsm), rest = each % warps;
+    return (double)(each / warps * (1 + warps) + (rest ? 1 + rest : 0)) * (chunks + 0.25);
+}
+
 // asynchronous dump files (output.cu): join the writer, free its buffers
 void dump_release(Ctx& c);
 

@@ -23,13 +23,9 @@ int sweep_lines(const Grid& g, int dir) {
     return dir == 0 && line_chunks<1>(g) <= 0.82 * line_chunks<kLines>(g) ? 1 : kLines;
 }
 
-// Length of the work items, in chunks: the one with the least time on the
-// busiest quarter of an SM, which holds `warps` warps at once.  A chunk takes
-// about 1 + w units of time with w warps beside one another (4.3k cycles alone
-// and 14k among three, FP64), and a segment's first five cells, which have no
-// interface yet, a quarter of a chunk.  Once no quarter gets a second item,
-// longer ones only take longer: the search ends there (at 2e6 cells in one line
-// trying every length takes 2 ms).
+// Length of the work items, in chunks: the one with the least sweep_time.  Once
+// no quarter of an SM gets a second item, longer ones only take longer: the
+// search ends there (at 2e6 cells in one line trying every length takes 2 ms).
 struct Plan { int chunks; long long each; };   // each: items per quarter of an SM
 template <int DIR, int NL>
 Plan pick_chunks(const Grid& g, int nsm, int warps) {
@@ -39,8 +35,8 @@ Plan pick_chunks(const Grid& g, int nsm, int warps) {
     Plan best{1, 0};
     double best_t = 0.0;
     for (int s = 1; s <= most; ++s) {
-        const long long each = (CUT(g, s).items() + 4 * nsm - 1) / (4 * nsm), rest = each % warps;
-        const double t = (double)(each / warps * (1 + warps) + (rest ? 1 + rest : 0)) * (s + 0.25);
+        const long long items = CUT(g, s).items(), each = (items + 4 * nsm - 1) / (4 * nsm);
+        const double t = sweep_time(items, s, nsm, warps);
         if (s == 1 || t < best_t) { best = Plan{s, each}; best_t = t; }
         if (each <= 1) break;
     }

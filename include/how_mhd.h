@@ -241,7 +241,9 @@ how_ctx* how_ensemble_member(how_ensemble* e, int m);
 int how_ensemble_init(how_ensemble* e);
 /* Sweep work-item shapes per direction (index into the candidate list of
  * how_ensemble_shape_info).  Without this call the first how_ensemble_run
- * autotunes: one real step per candidate, then the fastest per direction. */
+ * autotunes: one real step per candidate, then the fastest per direction.
+ * An ensemble with too few work items to fill the chip takes shorter ones (one
+ * chunk) than its shape's. */
 int how_ensemble_set_shapes(how_ensemble* e, int sx, int sy, int sz);
 int how_ensemble_get_shapes(const how_ensemble* e, int* shapes /*[3]*/, double* sweep_ms /*[3 x 3]*/);
 int how_ensemble_shape_info(int dir, int shape, int* lines, int* cells);

@@ -27,6 +27,7 @@ std::map<std::string, int> failing;                       // calls that fail, an
 std::vector<std::string> log_;                            // launches
 uintptr_t next_address = uintptr_t(1) << 40;
 int devices = 1;
+int watched = -1;                                         // offset into the first argument (fake_watch)
 thread_local int device = 0, last_error = kOk;
 thread_local bool capturing = false;
 thread_local struct { Dim grid, block; size_t smem; void* stream; } pushed;
@@ -52,6 +53,7 @@ void fake_reset(int ndevices) {
     std::lock_guard<std::mutex> l(mu);
     calls.clear(); failing.clear(); log_.clear();
     devices = ndevices;
+    watched = -1;
     device = 0;
     last_error = kOk;
 }
@@ -60,7 +62,10 @@ void fake_fail(const char* name, int error) {
     if (error) failing[name] = error; else failing.erase(name);
 }
 long fake_calls(const char* name) { std::lock_guard<std::mutex> l(mu); return calls[name]; }
-// the launches since the last call, a line each: captured, device, grid, block, dynamic shared memory, kernel
+// from here on launches of the sweeps note the int at this offset of their first argument
+void fake_watch(int offset) { watched = offset; }
+// the launches since the last call, a line each: captured, device, grid, block, dynamic shared memory, the
+// watched int, kernel
 const char* fake_launches() {
     static std::string out;
     std::lock_guard<std::mutex> l(mu);
@@ -88,15 +93,20 @@ int __cudaPopCallConfiguration(Dim* g, Dim* b, size_t* smem, void** stream) {
     *g = pushed.grid; *b = pushed.block; *smem = pushed.smem; *stream = pushed.stream;
     return 0;
 }
-int cudaLaunchKernel(const void* f, Dim g, Dim b, void**, size_t smem, void*) {
+int cudaLaunchKernel(const void* f, Dim g, Dim b, void** args, size_t smem, void*) {
     const int e = enter(capturing ? "captured launch" : "cudaLaunchKernel");
     if (e) return e;
     std::lock_guard<std::mutex> l(mu);
     const auto lim = smem_limit.find({device, f});
     if (smem > size_t(lim == smem_limit.end() ? 49152 : lim->second)) return done(kInvalidValue);
     char line[160];
-    std::snprintf(line, sizeof(line), "%d %d %u,%u,%u %u,%u,%u %zu ", int(capturing), device, g.x, g.y, g.z, b.x, b.y, b.z, smem);
-    log_.push_back(line + names[f]);
+    const std::string& name = names[f];
+    int seen = 0;
+    if (watched >= 0 && name.find("k_sweep") != std::string::npos)
+        std::memcpy(&seen, static_cast<char*>(args[0]) + watched, sizeof(int));
+    std::snprintf(line, sizeof(line), "%d %d %u,%u,%u %u,%u,%u %zu %d ", int(capturing), device, g.x, g.y, g.z, b.x, b.y,
+                  b.z, smem, seen);
+    log_.push_back(line + name);
     return kOk;
 }
 int cudaFuncSetAttribute(const void* f, int attr, int value) {

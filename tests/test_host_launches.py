@@ -60,8 +60,8 @@ def _params(hm, n, bc="periodic", **kw):
 
 class Launch:
     def __init__(self, row):
-        captured, device, grid, block, smem, self.kernel = row.split(" ", 5)
-        self.captured, self.device, self.smem = captured == "1", int(device), int(smem)
+        captured, device, grid, block, smem, watched, self.kernel = row.split(" ", 6)
+        self.captured, self.device, self.smem, self.watched = captured == "1", int(device), int(smem), int(watched)
         self.blocks = int(grid.split(",")[0])
 
 
@@ -211,6 +211,35 @@ def test_sweeps_of_few_lines_leave_no_lane_idle(lib, kw):
             d.ssprk(1e-3)
             x = _launches(fake, "k_sweepILi0E")
             assert len(x) == 5 and all("k_sweepILi0ELi%dE" % lines in r.kernel for r in x)
+
+
+@pytest.fixture(scope="module")
+def chunks_offset(tmp_path_factory):
+    """Where a sweep's arguments hold the chunks of its work items."""
+    d = tmp_path_factory.mktemp("offset")
+    (d / "o.cpp").write_text('#include "how_internal.cuh"\n#include <cstddef>\n#include <cstdio>\n'
+                             'int main() { std::printf("%d", (int)offsetof(how::SweepArgs, seg_chunks)); }\n')
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not found")
+    subprocess.run(["nvcc", "-x", "cu", "-std=c++17", "-w", "-I", str(PKG / "csrc"), "-I", str(PKG.parent / "include"),
+                    "-o", str(d / "o"), str(d / "o.cpp")], check=True)
+    return int(subprocess.run([str(d / "o")], check=True, capture_output=True, text=True).stdout)
+
+
+def test_small_ensembles_take_short_items(lib, chunks_offset):
+    """Members with too few items to fill the chip take items of one chunk, others
+    the shape's."""
+    hm, fake = lib
+    for n, members, chunks in ((200, 3, (1, 1, 1)), (200, 32, (1, 1, 1)), (64, 200, (2, 1, 1)), (20000, 16, (2, 8, 2))):
+        with hm.Ensemble([_params(hm, (n, 1, 1))] * members) as e:
+            e.init()
+            for shape in range(3):
+                e.set_shapes(shape, shape, shape)
+                _launches(fake)
+                fake.fake_watch(chunks_offset)
+                e.run(1)
+                x = _launches(fake, "k_sweep")
+                assert len(x) == 5 and all(r.watched == chunks[shape] for r in x)
 
 
 def test_cutting_a_long_line_takes_no_time(lib):
