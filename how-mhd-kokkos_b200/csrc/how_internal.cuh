@@ -174,7 +174,7 @@ struct Ctx {
     Grid g;
     int dev = 0;
     int sm_count = 148;             // of the device
-    SmemLimits smem;
+    SmemLimits smem;                // raised for this context's sweeps
     cudaStream_t stream = nullptr;
     double* mem = nullptr;          // one allocation for every field
     size_t mem_bytes = 0;

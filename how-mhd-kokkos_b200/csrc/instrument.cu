@@ -98,7 +98,7 @@ int how_get_kernel_timing(how_ctx* cp, double* total_ms, long* launches) {
 // Per-phase cycle accounting of one directional sweep of stage 1 (the
 // how_sweep semantics): out[k] = mean cycles a warp spends in phase k of a
 // chunk (0 load, 1 cell, 8 face, 9 CT terms, 10 update), measured by each
-// warp's first lane with clock64; out[11] = chunks.
+// warp's first lane with clock(); out[11] = chunks.
 int how_sweep_phase_profile(how_ctx* cp, int dir, double dt, double* out, int nout) {
     Ctx* c = cp;
     if (!c || !out) return HOW_ERR_ARG;

@@ -695,8 +695,10 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     volatile long long* sSpot = reinterpret_cast<long long*>(sm + M::bS) + lane;
 
     // tensor memory: a warp reaches lanes 32 (warp % 4) on, and the warps that
-    // share them take columns of their own.  (A kernel that allocates tensor
-    // memory runs one block per SM, so the block holds all of the SM's warps.)
+    // share them take columns of their own.  (The runtime's occupancy calculator
+    // answers one block per SM for this kernel with blocks of four warps too, whose
+    // registers and shared memory allow more, and a sweep then takes 4.1 ms: the
+    // block holds all of the SM's warps.)
     static_assert(WPB % 4 == 0, "blocks of whole tensor memory lanes");
     constexpr int kValues = 50, kPer = (kValues * (int)sizeof(R) / 4 + 3) / 4 * 4;   // columns per warp
     constexpr int kUsed = WPB / 4 * kPer, kColumns = kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
@@ -717,8 +719,8 @@ __global__ void __launch_bounds__(32 * WPB, MINB) k_sweep(const __grid_constant_
     // before the first, with the five cells before the first interface, has no
     // interface yet).  FP64 at 12 warps keeps it in shared memory and reads it
     // again where it is used: held across a chunk it takes 15 of 168 registers
-    // (256^3 sweep 3.05 ms with it, 2.54 without; the mixed method has them to
-    // spare, 0.85 against 0.89 ms at 192^3).
+    // (256^3 sweep 2.55 ms with it, 2.45 without; the mixed method has them to
+    // spare, 0.76 against 0.79 ms at 192^3).
     struct Place { int fb, fend, lo, t1_0, t2, item; const SweepArgs* a; };
     constexpr bool FREE_REGS = sizeof(R) == 4 || WPB <= 8;
     __shared__ Place s_place[FREE_REGS ? 1 : WPB];

@@ -10,8 +10,8 @@ namespace {
 
 // Lines per warp: four, whose rows are 32 bytes in y and z.  An x sweep takes one
 // line per warp, in chunks of 32 cells, where that makes 18% less chunks of
-// the domain, that is where lanes would be left without a line (1, 2, 3, 5, 6 or
-// 9 lines a plane, not too short).  FP64 x sweep with four lines and with one:
+// the domain, that is where lanes would be left without a line (1, 2, 3, 5, 6,
+// 9 lines a plane, on long lines 13).  FP64 x sweep with four lines and with one:
 // 1e5 cells of one line 75 and 26 us, 1024 x 1 x 1024 623 and 168, 1024 x 3 x 400
 // 279 and 201, 1024 x 5 x 200 280 and 164; 96^3, where no lane is idle, 186 and 191.
 constexpr int kLines = 4;
@@ -163,9 +163,9 @@ void launch_sweep(Ctx& c, int dir, const SweepArgs& a_in) {
     // instantiations: {fp64, mixed} x {plain, learned, guard-only}; label
     // collection runs the FP64 method.  Template arguments: warps per SM, whose
     // number caps the registers, and the warps of small domains.  FP64 at 12
-    // (168 registers): 2.54 ms per 256^3 sweep, against 2.64 at 8 (246); small
-    // domains at 8, whose chunk is shorter: 128^2 15.0 against 15.6 us.  Mixed at 12
-    // (168 registers): 0.85 ms per 192^3 sweep, against 1.01 at 8.
+    // (168 registers): 2.45 ms per 256^3 sweep, against 2.63 at 8 (250); small
+    // domains at 8, whose chunk is shorter: 128^2 14.9 against 15.6 us.  Mixed at 12
+    // (168 registers): 0.76 ms per 192^3 sweep, against 0.89 at 8.
 #define HOW_SWEEP_CASES(D)                                                  \
     do {                                                                    \
         if (mode == 3) { launch_one<D, 8, 0, double, 3>(c, a); break; }     \

@@ -26,14 +26,6 @@ __device__ __forceinline__ void tmem_wait_stores() { asm volatile("tcgen05.wait:
 template <int N> __device__ __forceinline__ void tmem_store(uint32_t at, const uint32_t* v);
 template <int N> __device__ __forceinline__ void tmem_load(uint32_t at, uint32_t* v);
 
-template <> __device__ __forceinline__ void tmem_store<1>(uint32_t at, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};"
-                 ::"r"(at), "r"(v[0]) : "memory");
-}
-template <> __device__ __forceinline__ void tmem_load<1>(uint32_t at, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];"
-                 : "=r"(v[0]) : "r"(at) : "memory");
-}
 template <> __device__ __forceinline__ void tmem_store<2>(uint32_t at, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};"
                  ::"r"(at), "r"(v[0]), "r"(v[1]) : "memory");
@@ -42,10 +34,6 @@ template <> __device__ __forceinline__ void tmem_load<2>(uint32_t at, uint32_t* 
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];"
                  : "=r"(v[0]), "=r"(v[1]) : "r"(at) : "memory");
 }
-template <> __device__ __forceinline__ void tmem_store<4>(uint32_t at, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
-                 ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-}
 template <> __device__ __forceinline__ void tmem_load<4>(uint32_t at, uint32_t* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
@@ -53,14 +41,6 @@ template <> __device__ __forceinline__ void tmem_load<4>(uint32_t at, uint32_t* 
 template <> __device__ __forceinline__ void tmem_store<8>(uint32_t at, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-template <> __device__ __forceinline__ void tmem_load<8>(uint32_t at, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(at) : "memory");
-}
-template <> __device__ __forceinline__ void tmem_store<16>(uint32_t at, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
 // The registers of the loads before are defined from here on: the values pass
 // through, so that no use moves ahead of the wait.
