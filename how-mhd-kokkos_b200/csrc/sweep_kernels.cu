@@ -9,9 +9,10 @@ namespace how {
 namespace {
 
 // Lines per warp: four, whose rows are 32 bytes in y and z.  An x sweep takes one
-// line per warp, in chunks of 32 cells, where that makes 18% less chunks of
-// the domain, that is where lanes would be left without a line (1, 2, 3, 5, 6,
-// 9 lines a plane, on long lines 13).  FP64 x sweep with four lines and with one:
+// line per warp, in chunks of 32 cells, where that makes 19% less chunks of
+// the domain, that is where lanes would be left without a line (1, 2, 3, 5, 6 or
+// 9 lines a plane; 13 give 18.7% at best and lost 2% of a 4096 x 13 step).  FP64
+// x sweep with four lines and with one:
 // 1e5 cells of one line 75 and 26 us, 1024 x 1 x 1024 623 and 168, 1024 x 3 x 400
 // 279 and 201, 1024 x 5 x 200 280 and 164; 96^3, where no lane is idle, 186 and 191.
 constexpr int kLines = 4;
@@ -20,7 +21,7 @@ template <int NL> double line_chunks(const Grid& g) {   // of a plane, with a qu
     return CUT(g, 1).groups * ((g.nx - CUT::f0) / CUT::W + 1.25);
 }
 int sweep_lines(const Grid& g, int dir) {
-    return dir == 0 && line_chunks<1>(g) <= 0.82 * line_chunks<kLines>(g) ? 1 : kLines;
+    return dir == 0 && line_chunks<1>(g) <= 0.81 * line_chunks<kLines>(g) ? 1 : kLines;
 }
 
 // Length of the work items, in chunks: the one with the least sweep_time.  Once

@@ -204,8 +204,9 @@ def test_a_launch_refused_in_a_capture_is_not_left_out(lib):
 def test_sweeps_of_few_lines_leave_no_lane_idle(lib, kw):
     """x sweeps of one, two, three, five lines a plane: a line per warp; else four."""
     hm, fake = lib
-    for n, lines in (((40000, 1, 1), 1), ((300, 1, 300), 1), ((300, 3, 1), 1), ((300, 5, 20), 1), ((5, 5, 300), 4),
-                     ((300, 4, 1), 4), ((300, 7, 1), 4), ((300, 300, 1), 4), ((40, 40, 40), 4)):
+    for n, lines in (((40000, 1, 1), 1), ((300, 1, 300), 1), ((300, 3, 1), 1), ((300, 5, 20), 1), ((4096, 9, 1), 1),
+                     ((5, 5, 300), 4), ((300, 4, 1), 4), ((300, 7, 1), 4), ((4096, 13, 1), 4), ((300, 300, 1), 4),
+                     ((40, 40, 40), 4)):
         with hm.Domain(_params(hm, n, **kw)) as d:
             _launches(fake)
             d.ssprk(1e-3)
